@@ -15,9 +15,10 @@ namespace nb {
 constexpr int kDiagThreads = 256;
 constexpr int kDiagVals = 12;  // KE, Px, Py, Pz, Lx, Ly, Lz, Mx, My, Mz, M, PE
 
-// Block partial sums of the per-body terms (fixed shuffle-tree order).
+// Block partial sums of the per-body terms (fixed shuffle-tree order).  phi
+// (may be null): the tree potential by row; the PE terms are 1/2 m_i phi_i.
 __global__ void __launch_bounds__(kDiagThreads)
-k_diag_partials(int n, State s, const double* __restrict__ pe_terms, double* __restrict__ part) {
+k_diag_partials(int n, State s, const double* __restrict__ phi, double* __restrict__ part) {
     __shared__ double sh[kDiagVals][kDiagThreads / 32];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double v[kDiagVals];
@@ -35,7 +36,7 @@ k_diag_partials(int n, State s, const double* __restrict__ pe_terms, double* __r
         v[6] = x * mvy - y * mvx;
         v[7] = m * x; v[8] = m * y; v[9] = m * z;
         v[10] = m;
-        v[11] = pe_terms ? pe_terms[i] : 0.0;
+        v[11] = phi ? 0.5 * m * phi[i] : 0.0;
     }
 #pragma unroll
     for (int k = 0; k < kDiagVals; k++) v[k] = warp_sum(v[k]);
@@ -51,61 +52,146 @@ k_diag_partials(int n, State s, const double* __restrict__ pe_terms, double* __r
     }
 }
 
-__global__ void k_diag_final(int nblocks, const double* __restrict__ part, double* __restrict__ out) {
-    // thread k sums column k over the blocks in block order
-    if (threadIdx.x >= kDiagVals) return;
+// Block k sums column k over the partials (thread-strided, then a fixed
+// shuffle tree: deterministic); block 11 adds the pair-sum items too.  One
+// thread per column walking the blocks one load after another took 17.6 us
+// at 65,537 bodies, and 16 times that at 2^20.
+__global__ void __launch_bounds__(kDiagThreads)
+k_diag_final(int nblocks, const double* __restrict__ part, int n_items,
+             const double* __restrict__ items, double* __restrict__ out) {
+    __shared__ double sh[kDiagThreads / 32];
+    const int k = blockIdx.x;
     double t = 0.0;
-    for (int b = 0; b < nblocks; b++) t += part[(size_t)b * kDiagVals + threadIdx.x];
-    out[threadIdx.x] = t;
+    for (int b = threadIdx.x; b < nblocks; b += kDiagThreads) t += part[(size_t)b * kDiagVals + k];
+    if (k == kDiagVals - 1)
+        for (int b = threadIdx.x; b < n_items; b += kDiagThreads) t += items[b];
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        t = 0.0;
+        for (int w = 0; w < kDiagThreads / 32; w++) t += sh[w];
+        out[k] = t;
+    }
 }
 
-// Exact pair potential: row i holds sum_{j>i, active} -m_i m_j / sqrt(r^2+eps^2).
-__global__ void k_pe_rows(int n, State s, double eps2, double* __restrict__ rows) {
-    __shared__ double4 sj[128];
-    __shared__ uint8_t sa[128];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool me = i < n && s.active[i];
-    const double xi = me ? s.px[i] : 0, yi = me ? s.py[i] : 0, zi = me ? s.pz[i] : 0;
-    const double mi = me ? s.mass[i] : 0;
-    double acc = 0.0;
-    const int start = blockIdx.x * blockDim.x;
-    for (int base = start; base < n; base += 128) {
+// 1/sqrt(x) in FP64 from the hardware's approximation on the high word
+// (rsqrt.approx.ftz.f64: relative error at most 2^-20.0 over 2^32 arguments
+// spread over [1, 4)) and one third-order Householder step,
+// y <- y (1 + e/2 + 3e^2/8) with e = 1 - x y^2, which cubes the relative error
+// (2^-58 before FP64 rounding).  x = 0, subnormal, infinite or NaN takes
+// the library routine.
+__device__ __forceinline__ double rsqrt_f64(double x) {
+    if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) return rsqrt(x);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// Exact pair potential, sum over active pairs i < j of
+// -m_i m_j / sqrt(r^2 + eps^2), as a grid of (tile of 512 rows, chunk of
+// sources) items that lie on or above the diagonal: each thread holds two
+// rows, the sources are staged 256 at a time in shared memory (two broadcast
+// reads for two pairs) and each item's sum goes to out[chunk * tiles + tile]
+// (items below the diagonal write 0).  About 12 FP64 operations a pair bound
+// it.  The chunk length gives some 16 useful items per SM, so the triangle
+// fills the GPU evenly; one thread per row over all later rows, with a
+// correctly rounded square root and division per pair, left the first rows'
+// blocks running alone.  A whole diagnostics call, before -> now: 2,000
+// bodies 444 -> 57 us, 65,537 bodies 13.39 -> 2.06 ms, 131,072 bodies 29.3 ->
+// 8.2 ms (the FP64 pipe is 71 % busy; 1, 3 and 4 rows per thread were within 5 %).
+constexpr int kPeThreads = 256;
+constexpr int kPeRows = 2;                        // rows per thread
+constexpr int kPeTile = kPeThreads * kPeRows;     // rows per item
+constexpr int kPeStage = 256;                     // sources staged at a time
+constexpr int kPeMinChunk = 64;
+
+__global__ void __launch_bounds__(kPeThreads)
+k_pe_items(int n, State s, double eps2, int chunk, double* __restrict__ out) {
+    __shared__ double4 sj[kPeStage];
+    __shared__ double sh[kPeThreads / 32];
+    const int i0 = blockIdx.x * kPeTile;
+    const int j0 = max(i0, (int)blockIdx.y * chunk);
+    const int j1 = min(n, ((int)blockIdx.y + 1) * chunk);
+    double acc[kPeRows], xi[kPeRows], yi[kPeRows], zi[kPeRows], mi[kPeRows];
+    int row[kPeRows];
+#pragma unroll
+    for (int u = 0; u < kPeRows; u++) {
+        const int i = i0 + u * kPeThreads + threadIdx.x;
+        const bool me = i < n && s.active[i];
+        row[u] = me ? i : n;  // no source lies above row n
+        xi[u] = me ? s.px[i] : 0.0;
+        yi[u] = me ? s.py[i] : 0.0;
+        zi[u] = me ? s.pz[i] : 0.0;
+        mi[u] = me ? s.mass[i] : 0.0;
+        acc[u] = 0.0;
+    }
+    for (int base = j0; base < j1; base += kPeStage) {
         const int j = base + threadIdx.x;
-        sj[threadIdx.x] = (j < n) ? make_double4(s.px[j], s.py[j], s.pz[j], s.mass[j]) : make_double4(0, 0, 0, 0);
-        sa[threadIdx.x] = (j < n) ? s.active[j] : 0;
+        // an inactive source is massless and far away (finite: its term is 0)
+        if (threadIdx.x < kPeStage)
+            sj[threadIdx.x] = j < j1 && s.active[j]
+                                  ? make_double4(s.px[j], s.py[j], s.pz[j], s.mass[j])
+                                  : make_double4(1e150, 0.0, 0.0, 0.0);
         __syncthreads();
-        if (me) {
-            const int cnt = min(128, n - base);
+        const int cnt = min(kPeStage, j1 - base);
+        // above the tile's rows every source counts for every active row
+        if (base >= i0 + kPeTile) {
+#pragma unroll 4
             for (int k = 0; k < cnt; k++) {
-                if (base + k <= i || !sa[k]) continue;
                 const double4 q = sj[k];
-                const double rx = q.x - xi, ry = q.y - yi, rz = q.z - zi;
-                const double d2 = rx * rx + ry * ry + rz * rz + eps2;
-                acc += -1.0 * mi * q.w / sqrt(d2);
+#pragma unroll
+                for (int u = 0; u < kPeRows; u++) {
+                    const double dx = q.x - xi[u], dy = q.y - yi[u], dz = q.z - zi[u];
+                    acc[u] = fma(q.w, rsqrt_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), acc[u]);
+                }
+            }
+        } else {
+            for (int k = 0; k < cnt; k++) {
+                const double4 q = sj[k];
+#pragma unroll
+                for (int u = 0; u < kPeRows; u++) {
+                    if (base + k <= row[u]) continue;
+                    const double dx = q.x - xi[u], dy = q.y - yi[u], dz = q.z - zi[u];
+                    acc[u] = fma(q.w, rsqrt_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), acc[u]);
+                }
             }
         }
         __syncthreads();
     }
-    if (i < n) rows[i] = acc;
-}
-
-// 1/2 m_i phi_i terms from the tree potential.
-__global__ void k_pe_from_phi(int n, State s, const double* __restrict__ phi, double* __restrict__ rows) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    rows[i] = s.active[i] ? 0.5 * s.mass[i] * phi[i] : 0.0;
+    double t = 0.0;
+#pragma unroll
+    for (int u = 0; u < kPeRows; u++)
+        if (row[u] < n) t -= mi[u] * acc[u];
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        t = 0.0;
+        for (int w = 0; w < kPeThreads / 32; w++) t += sh[w];
+        out[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
+    }
 }
 
 void diagnostics(cudaStream_t st, int n, const State& s, double eps, int pe_mode,
-                 const double* phi, double* rows, double* part, double* out12) {
+                 const double* phi, double* items, double* part, double* out12) {
     const int nb = ceil_div(n > 0 ? n : 1, kDiagThreads);
-    if (pe_mode == 0) {
-        if (n > 0) k_pe_rows<<<ceil_div(n, 128), 128, 0, st>>>(n, s, eps * eps, rows);
-    } else {
-        if (n > 0) k_pe_from_phi<<<ceil_div(n, 256), 256, 0, st>>>(n, s, phi, rows);
+    int n_items = 0;
+    if (n > 0 && pe_mode == 0) {
+        const int tiles = ceil_div(n, kPeTile);
+        // half of the items are useful (the triangle).  They are at most n,
+        // which is what `items` holds: tiles * ceil(n / 64) <= n up to 16,384
+        // rows, and tiles + 32 kSMs <= n from there on
+        const int want = ceil_div(32 * kSMs, tiles);
+        const int chunks = std::max(1, std::min(want, ceil_div(n, kPeMinChunk)));
+        const int chunk = ceil_div(ceil_div(n, chunks), kPeMinChunk) * kPeMinChunk;
+        const dim3 grid(tiles, ceil_div(n, chunk));
+        n_items = (int)(grid.x * grid.y);
+        k_pe_items<<<grid, kPeThreads, 0, st>>>(n, s, eps * eps, chunk, items);
     }
-    if (n > 0) k_diag_partials<<<nb, kDiagThreads, 0, st>>>(n, s, rows, part);
-    k_diag_final<<<1, 32, 0, st>>>(n > 0 ? nb : 0, part, out12);
+    if (n > 0) k_diag_partials<<<nb, kDiagThreads, 0, st>>>(n, s, pe_mode == 0 ? nullptr : phi, part);
+    k_diag_final<<<kDiagVals, kDiagThreads, 0, st>>>(n > 0 ? nb : 0, part, n_items, items, out12);
 }
 
 size_t diag_partial_bytes(int capacity) {
@@ -123,17 +209,6 @@ size_t diag_partial_bytes(int capacity) {
 // summed in chunk order, so the result is deterministic.
 constexpr int kTgtTile = 8;
 
-// 1/sqrt(x) in FP64 from the FP32 hardware estimate (relative error below
-// 2^-22) and one third-order Householder step, y <- y (1 + e/2 + 3e^2/8)
-// with e = 1 - x y^2, which cubes the relative error (below 2^-64, so the
-// result is within FP64 rounding).  x outside [1e-36, 1e36] (beyond the
-// FP32 normal range after conversion) takes the library routine.
-__device__ __forceinline__ double rsqrt_f64(double x) {
-    if (!(x >= 1e-36 && x <= 1e36)) return rsqrt(x);
-    const double y = (double)rsqrt_ftz((float)x);
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
 constexpr int kTgtThreads = 256;
 constexpr int kTgtUnroll = 4;
 constexpr int kTgtMinChunk = 16384;

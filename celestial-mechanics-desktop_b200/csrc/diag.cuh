@@ -8,8 +8,9 @@ namespace nb {
 size_t diag_partial_bytes(int capacity);
 // out12: KE, Px, Py, Pz, Lx, Ly, Lz, sum m x, sum m y, sum m z, M, PE.
 // pe_mode 0: exact pair sum; 1: 1/2 sum m_i phi_i from `phi` (by row).
+// items: scratch of n doubles.
 void diagnostics(cudaStream_t st, int n, const State& s, double eps, int pe_mode,
-                 const double* phi, double* rows, double* part, double* out12);
+                 const double* phi, double* items, double* part, double* out12);
 // FP64 direct-sum accelerations of rows targets[0 .. nt) into out3 (xyz per
 // target); scratch: direct_targets_scratch_bytes(sms).
 size_t direct_targets_scratch_bytes(int sms);
