@@ -297,13 +297,31 @@ __global__ void k_direct_reduce(int n, int chunks, const double* __restrict__ pa
     az[row] = s[2];
 }
 
-// The arithmetic is split in two phases so that the costly per-pair part
-// (sqrt, division) runs on every thread of the block: for a tile of kPTj
-// sources, 256 threads compute the kPTi x kPTj pair terms c*dx, c*dy, c*dz
-// (each rounded exactly as above) into shared memory; then 3 x kPTi threads
-// subtract them in source order, one (target, component) chain per thread.
-// The sequence of roundings of every target's sum is unchanged, so the
-// result is bit-identical to CpuParallelBackend's.
+// The FP64 pair sum.  Every target's terms have to be subtracted one by one
+// in source order (that order is what makes the result bit-identical to
+// CpuParallelBackend's), so a target component is one chain of n dependent
+// additions; the costly part of a term (a correctly rounded square root and
+// division) is not part of the chain.  A block therefore has producer warps,
+// which compute the TI x kPTj pair terms of a source tile (each rounded
+// exactly as the CPU code rounds it) into one of two shared-memory buffers,
+// and one accumulator warp, whose lane (target, component) walks the other
+// buffer meanwhile: one barrier a tile, and the chain and the term arithmetic
+// overlap.  A term that is not added (the body itself, an inactive source) is
+// stored as +0, whose subtraction changes no bit.  The chain bounds a small
+// system (1000 dependent additions), the square root and division a large
+// one; the two buffers are 2 x 25 KB at TI = 8, so two blocks share an SM.
+// Two phases of a tile behind one another, 256 threads for both, took 51.2 us
+// for 1,000 bodies, 731 us for 8,192 and 3.47 ms for 20,000; now 21.5, 273 and
+// 1,424 us (call times on the stream; 10, 53 and 60 % of the FP64 rate by some
+// 40 operations a pair).  Half the tile (64 sources) was 17 to 28 % slower.
+//
+// A step of the integrator needs nothing else: the accumulator lane that ends
+// with component c of a body's acceleration closes the step (v += dt/2 a) and
+// opens the next one (v += dt'/2 a, x' = x + dt' v, in the order and rounding
+// of SoAVerletIntegrator.Step), writing x' to the other position buffer, since
+// other blocks may still read x.  One launch a step, each started while its
+// predecessor ends, instead of three and four memsets: 1,000 bodies 43.3 ->
+// 11.0 us a step, 200 bodies 20.7 -> 4.9, 3,000 bodies 117 -> 43.8.
 //
 // ORDER selects the rounding and summation order of another CPU backend of
 // the desktop app (without the shell theorem; with it every backend runs
@@ -318,117 +336,268 @@ __global__ void k_direct_reduce(int n, int chunks, const double* __restrict__ pa
 //                   body's sum is (its running sum over lower rows, which the
 //                   loop adds into ax[j] as +c*(x_lower - x_j), i.e. minus
 //                   the term) + (its running sum over higher rows).
-constexpr int kPTi = 8;     // targets per block
-constexpr int kPTj = 128;   // sources per tile
-constexpr int kPThreads = 256;
+constexpr int kPTj = 128;        // sources per tile
+constexpr int kPRow = kPTj + 2;  // padded row: the lanes' 16-byte reads meet no bank twice
 
-template <bool SHELL, int ORDER>
-__global__ void __launch_bounds__(kPThreads)
-k_direct_fp64_pairs(int n, const double* __restrict__ px, const double* __restrict__ py,
-                    const double* __restrict__ pz, const double* __restrict__ m,
-                    const double* __restrict__ rad, const uint8_t* __restrict__ act,
-                    double eps2, double* __restrict__ ax, double* __restrict__ ay,
-                    double* __restrict__ az) {
-    __shared__ double s_t[3][kPTi][kPTj + 1];  // pair terms (padded against bank conflicts)
-    __shared__ uint8_t s_ok[kPTi][kPTj];        // term is added (active source, not self)
-    __shared__ double s_i[kPTi][3];
-    __shared__ uint8_t s_iact[kPTi];
-    const int i0 = blockIdx.x * kPTi;
-    if (threadIdx.x < kPTi) {
+template <int TI, bool MANY>
+struct Fp64Shape {
+    // producer threads: one block per SM (not MANY) hides the term's latency
+    // with threads, several blocks with independent terms per thread
+    static constexpr int most = MANY ? 256 : 512;
+    static constexpr int producers = TI * kPTj < most ? TI * kPTj : most;
+    static constexpr int threads = 32 + producers;
+    static constexpr int blocks = MANY ? 3 : 1;
+    static constexpr size_t smem = sizeof(double) * 2 * 3 * TI * kPRow;
+};
+
+template <bool SHELL, int ORDER, int TI, bool MANY>
+__global__ void __launch_bounds__(Fp64Shape<TI, MANY>::threads, Fp64Shape<TI, MANY>::blocks)
+k_direct_fp64_pairs(Fp64Args a) {
+    constexpr int kProd = Fp64Shape<TI, MANY>::producers;
+    constexpr int kPer = TI * kPTj / kProd;  // terms per producer thread and tile
+    static_assert(kProd % kPTj == 0 && kPer * kProd == TI * kPTj && 3 * TI <= 32, "block shape");
+    extern __shared__ __align__(16) double s_t[];  // [2][3 TI][kPRow]
+    __shared__ double s_i[TI][3];
+    __shared__ uint8_t s_iact[TI];
+    // the previous step's kernel has ended, and its stores are visible (a
+    // launch without the overlap attribute passes at once)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int n = a.n;
+    const int i0 = blockIdx.x * TI;
+    if (threadIdx.x < TI) {
         const int i = i0 + threadIdx.x;
-        const bool me = i < n && act[i];
+        const bool me = i < n && a.act[i];
+        const double x = me ? a.px[i] : 0.0, y = me ? a.py[i] : 0.0, z = me ? a.pz[i] : 0.0;
         s_iact[threadIdx.x] = me;
-        s_i[threadIdx.x][0] = me ? px[i] : 0.0;
-        s_i[threadIdx.x][1] = me ? py[i] : 0.0;
-        s_i[threadIdx.x][2] = me ? pz[i] : 0.0;
+        s_i[threadIdx.x][0] = x;
+        s_i[threadIdx.x][1] = y;
+        s_i[threadIdx.x][2] = z;
+        if (me && !(isfinite(x) && isfinite(y) && isfinite(z) && isfinite(a.m[i])))
+            dev_flag(a.err, kErrNonFinite);
     }
     __syncthreads();
-    // accumulator thread: (target, component)
-    const int acc_t = threadIdx.x / 3, acc_c = threadIdx.x % 3;
-    const bool accum = threadIdx.x < 3 * kPTi;
+    const int tiles = (n + kPTj - 1) / kPTj;
     constexpr bool kSplit = !SHELL && ORDER == kOrderPairwise;
+    if (threadIdx.x >= 32) {
+        // producer: source column tj of every tile, targets ti0, ti0 + kProd / kPTj, ...
+        const int p = threadIdx.x - 32;
+        const int tj = p % kPTj, ti0 = p / kPTj;
+        double xj = 0.0, yj = 0.0, zj = 0.0, mj = 0.0, R = 0.0;
+        bool aj = false;
+        auto load = [&](int j) {
+            aj = j < n && a.act[j];
+            if (aj) {
+                xj = a.px[j];
+                yj = a.py[j];
+                zj = a.pz[j];
+                mj = a.m[j];
+                if (SHELL) R = a.rad[j];
+            }
+        };
+        load(tj);
+        for (int t = 0; t <= tiles; t++) {
+            if (t < tiles) {
+                const int j = t * kPTj + tj;
+                const double cx = xj, cy = yj, cz = zj, cm = mj, cR = R;
+                const bool ca = aj;
+                load(j + kPTj);  // the next tile's words travel while this one is computed
+                double* out = s_t + (t & 1) * (3 * TI * kPRow) + tj;
+#pragma unroll
+                for (int k = 0; k < kPer; k++) {
+                    const int ti = ti0 + k * (kProd / kPTj);
+                    double tx = 0.0, ty = 0.0, tz = 0.0;
+                    if (ca && j != i0 + ti) {
+                        const double dx = __dsub_rn(s_i[ti][0], cx);
+                        const double dy = __dsub_rn(s_i[ti][1], cy);
+                        const double dz = __dsub_rn(s_i[ti][2], cz);
+                        const double raw = __dadd_rn(
+                            __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+                        double c;
+                        if (SHELL && cR > 0.0 && sqrt(raw) < cR) {
+                            const double den = __dadd_rn(__dmul_rn(cR, cR), a.eps2);
+                            const double ids = 1.0 / sqrt(den);
+                            c = __dmul_rn(cm, ids) / den;
+                        } else {
+                            const double inv = 1.0 / sqrt(__dadd_rn(raw, a.eps2));
+                            c = !SHELL && ORDER != kOrderParallel
+                                    ? __dmul_rn(cm, __dmul_rn(__dmul_rn(inv, inv), inv))
+                                    : __dmul_rn(__dmul_rn(__dmul_rn(cm, inv), inv), inv);
+                        }
+                        tx = __dmul_rn(c, dx);
+                        ty = __dmul_rn(c, dy);
+                        tz = __dmul_rn(c, dz);
+                    }
+                    out[(3 * ti + 0) * kPRow] = tx;
+                    out[(3 * ti + 1) * kPRow] = ty;
+                    out[(3 * ti + 2) * kPRow] = tz;
+                }
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    // accumulator lane: (target, component)
+    const int lane = threadIdx.x < 3 * TI ? threadIdx.x : 0;
+    const int acc_t = lane / 3, acc_c = lane % 3;
+    const int i = i0 + acc_t;
     double sum = 0.0;
     double hi = 0.0;  // kSplit: the sum over higher rows (sum holds the lower rows')
-    for (int base = 0; base < n; base += kPTj) {
-        for (int p = threadIdx.x; p < kPTi * kPTj; p += kPThreads) {
-            const int ti = p / kPTj, tj = p % kPTj;
-            const int i = i0 + ti, j = base + tj;
-            bool ok = j < n && s_iact[ti] && j != i && act[j];
-            double tx = 0.0, ty = 0.0, tz = 0.0;
-            if (ok) {
-                const double dx = __dsub_rn(s_i[ti][0], px[j]);
-                const double dy = __dsub_rn(s_i[ti][1], py[j]);
-                const double dz = __dsub_rn(s_i[ti][2], pz[j]);
-                const double raw = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                             __dmul_rn(dz, dz));
-                const double mj = m[j];
-                double c;
-                const double R = SHELL ? rad[j] : 0.0;
-                if (!SHELL && ORDER != kOrderParallel) {
-                    const double inv = 1.0 / sqrt(__dadd_rn(raw, eps2));
-                    c = __dmul_rn(mj, __dmul_rn(__dmul_rn(inv, inv), inv));
-                } else if (!SHELL || R <= 0.0) {
-                    const double inv = 1.0 / sqrt(__dadd_rn(raw, eps2));
-                    c = __dmul_rn(__dmul_rn(__dmul_rn(mj, inv), inv), inv);
-                } else if (sqrt(raw) < R) {
-                    const double den = __dadd_rn(__dmul_rn(R, R), eps2);
-                    const double ids = 1.0 / sqrt(den);
-                    c = __dmul_rn(mj, ids) / den;
-                } else {
-                    const double inv = 1.0 / sqrt(__dadd_rn(raw, eps2));
-                    c = __dmul_rn(__dmul_rn(__dmul_rn(mj, inv), inv), inv);
-                }
-                tx = __dmul_rn(c, dx);
-                ty = __dmul_rn(c, dy);
-                tz = __dmul_rn(c, dz);
-            }
-            s_t[0][ti][tj] = tx;
-            s_t[1][ti][tj] = ty;
-            s_t[2][ti][tj] = tz;
-            s_ok[ti][tj] = ok;
-        }
-        __syncthreads();
-        if (accum) {
+    for (int t = 0; t <= tiles; t++) {
+        if (t > 0) {
+            const int base = (t - 1) * kPTj;
+            const double2* row =
+                (const double2*)(s_t + ((t - 1) & 1) * (3 * TI * kPRow) + lane * kPRow);
             const int cnt = min(kPTj, n - base);
             if (kSplit) {
-                const int split = i0 + acc_t - base;  // first tj with j > i
+                const int split = i - base;  // first tj with j > i (the body's own term is 0)
+                const double* r = (const double*)row;
                 for (int tj = 0; tj < cnt; tj++) {
-                    if (!s_ok[acc_t][tj]) continue;
-                    if (tj < split) sum = __dsub_rn(sum, s_t[acc_c][acc_t][tj]);
-                    else hi = __dsub_rn(hi, s_t[acc_c][acc_t][tj]);
+                    if (tj < split) sum = __dsub_rn(sum, r[tj]);
+                    else hi = __dsub_rn(hi, r[tj]);
                 }
             } else {
-                for (int tj = 0; tj < cnt; tj++)
-                    if (s_ok[acc_t][tj]) sum = __dsub_rn(sum, s_t[acc_c][acc_t][tj]);
+                // rows past n were stored as 0
+                const int blocks = (cnt + 15) / 16;
+                for (int k = 0; k < blocks; k++) {
+                    double2 v[8];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) v[u] = row[8 * k + u];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        sum = __dsub_rn(sum, v[u].x);
+                        sum = __dsub_rn(sum, v[u].y);
+                    }
+                }
             }
         }
         __syncthreads();
     }
-    if (accum) {
-        const int i = i0 + acc_t;
-        if (kSplit) sum = __dadd_rn(sum, hi);
-        if (i < n) (acc_c == 0 ? ax : acc_c == 1 ? ay : az)[i] = sum;
+    if (threadIdx.x >= 3 * TI || i >= n) return;
+    const bool me = s_iact[acc_t];
+    if (kSplit) sum = __dadd_rn(sum, hi);
+    if (!me) sum = 0.0;
+    a.acc[acc_c][i] = sum;
+    if (!a.close && !a.open) return;
+    double v = 0.0;
+    if (me) {
+        v = a.vel[acc_c][i];
+        if (a.close) v = __dadd_rn(v, __dmul_rn(0.5 * a.dt_close, sum));
+        if (a.open) v = __dadd_rn(v, __dmul_rn(0.5 * a.dt_open, sum));
+        a.vel[acc_c][i] = v;
+    }
+    if (a.open) {
+        const double x = acc_c == 0 ? a.px[i] : acc_c == 1 ? a.py[i] : a.pz[i];
+        a.next[acc_c][i] = me ? __dadd_rn(x, __dmul_rn(a.dt_open, v)) : x;
     }
 }
 
-void direct_fp64(cudaStream_t st, int n, const double* px, const double* py, const double* pz,
-                 const double* m, const double* rad, const uint8_t* act, double eps, bool shell,
-                 int order, double* ax, double* ay, double* az) {
-    if (n <= 0) return;
-    const double eps2 = eps * eps;
-    const int g = ceil_div(n, kPTi);
-    if (shell)
-        k_direct_fp64_pairs<true, kOrderParallel><<<g, kPThreads, 0, st>>>(
-            n, px, py, pz, m, rad, act, eps2, ax, ay, az);
-    else if (order == kOrderSimd)
-        k_direct_fp64_pairs<false, kOrderSimd><<<g, kPThreads, 0, st>>>(
-            n, px, py, pz, m, rad, act, eps2, ax, ay, az);
-    else if (order == kOrderPairwise)
-        k_direct_fp64_pairs<false, kOrderPairwise><<<g, kPThreads, 0, st>>>(
-            n, px, py, pz, m, rad, act, eps2, ax, ay, az);
-    else
-        k_direct_fp64_pairs<false, kOrderParallel><<<g, kPThreads, 0, st>>>(
-            n, px, py, pz, m, rad, act, eps2, ax, ay, az);
+// Opens the first of a run of steps: v += dt/2 a, x' = x + dt v for active
+// rows, every row's position to `next` (which may be the position arrays).
+__global__ void k_fp64_open(Fp64Args a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n) return;
+    const bool me = a.act[i];
+    const double* const pos[3] = {a.px, a.py, a.pz};
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        double x = pos[c][i];
+        if (me) {
+            const double v = __dadd_rn(a.vel[c][i], __dmul_rn(0.5 * a.dt_open, a.acc[c][i]));
+            a.vel[c][i] = v;
+            x = __dadd_rn(x, __dmul_rn(a.dt_open, v));
+        }
+        a.next[c][i] = x;
+    }
+}
+
+namespace {
+
+template <bool SHELL, int ORDER, int TI, bool MANY>
+cudaError_t launch_fp64(cudaStream_t st, const Fp64Args& a) {
+    using Shape = Fp64Shape<TI, MANY>;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ceil_div(a.n, TI));
+    cfg.blockDim = dim3(Shape::threads);
+    cfg.dynamicSmemBytes = Shape::smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_direct_fp64_pairs<SHELL, ORDER, TI, MANY>, a);
+}
+
+template <bool SHELL, int ORDER, bool MANY>
+void init_fp64() {
+    cudaFuncSetAttribute((const void*)k_direct_fp64_pairs<SHELL, ORDER, 8, MANY>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)Fp64Shape<8, MANY>::smem);
+}
+
+template <int TI, bool MANY>
+cudaError_t launch_fp64_order(cudaStream_t st, const Fp64Args& a, bool shell, int order) {
+    if (shell) return launch_fp64<true, kOrderParallel, TI, MANY>(st, a);
+    if (order == kOrderSimd) return launch_fp64<false, kOrderSimd, TI, MANY>(st, a);
+    if (order == kOrderPairwise) return launch_fp64<false, kOrderPairwise, TI, MANY>(st, a);
+    return launch_fp64<false, kOrderParallel, TI, MANY>(st, a);
+}
+
+template <bool MANY>
+void init_fp64_orders() {
+    init_fp64<true, kOrderParallel, MANY>();
+    init_fp64<false, kOrderParallel, MANY>();
+    init_fp64<false, kOrderSimd, MANY>();
+    init_fp64<false, kOrderPairwise, MANY>();
+}
+
+}  // namespace
+
+void direct_init() {
+    init_fp64_orders<false>();
+    init_fp64_orders<true>();
+}
+
+// Targets per block: the fewest of 2, 4, 8 that still gives every block an SM
+// of its own (a block's chain takes as long for 2 targets as for 8, and its
+// terms take less); beyond that 8 targets, which share the source loads, in
+// smaller blocks with more independent terms per thread, several to an SM.
+// Measured at 8,192 bodies: 512 producers 460 us, 256 273, 128 276; at 1,000
+// bodies (8 targets, one block per SM) 512 producers 11.4 us a step, 256 12.2.
+cudaError_t direct_fp64(cudaStream_t st, const Fp64Args& a, bool shell, int order, int sms) {
+    if (a.n <= 0) return cudaSuccess;
+    if (ceil_div(a.n, 2) <= sms) return launch_fp64_order<2, false>(st, a, shell, order);
+    if (ceil_div(a.n, 4) <= sms) return launch_fp64_order<4, false>(st, a, shell, order);
+    if (ceil_div(a.n, 8) <= sms) return launch_fp64_order<8, false>(st, a, shell, order);
+    return launch_fp64_order<8, true>(st, a, shell, order);
+}
+
+// The opening kick-drift writes positions to the buffer from which the
+// alternation ends in pos[0], so the caller's arrays hold the final state.
+cudaError_t direct_fp64_steps(cudaStream_t st, Fp64Args a, bool shell, int order, int sms,
+                              double* const pos[2][3], const double* dts, int n_dt, int steps) {
+    if (a.n <= 0 || steps <= 0) return cudaSuccess;
+    int buf = (steps - 1) & 1;
+    auto use = [&](int from, int to) {
+        a.px = pos[from][0];
+        a.py = pos[from][1];
+        a.pz = pos[from][2];
+        for (int c = 0; c < 3; c++) a.next[c] = pos[to][c];
+    };
+    use(0, buf);
+    a.dt_open = dts[0];
+    k_fp64_open<<<ceil_div(a.n, 256), 256, 0, st>>>(a);
+    cudaError_t e = cudaPeekAtLastError();
+    for (int k = 0; k < steps && e == cudaSuccess; k++, buf ^= 1) {
+        use(buf, buf ^ 1);
+        a.close = true;
+        a.open = k + 1 < steps;
+        a.dt_close = dts[k % n_dt];
+        a.dt_open = dts[(k + 1) % n_dt];
+        e = direct_fp64(st, a, shell, order, sms);
+    }
+    return e;
 }
 
 void direct_fp32(cudaStream_t st, int n, const double4* sbody, const float* srad,

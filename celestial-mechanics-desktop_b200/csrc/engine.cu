@@ -260,6 +260,33 @@ void record(nb_engine* h, int k) {
     if (h->timing) cudaEventRecord(h->ev[k], h->st);
 }
 
+// The FP64 direct sum's arguments for the current device rows.
+nb::Fp64Args fp64_args(nb_engine* h, double eps) {
+    nb::Fp64Args a{};
+    a.n = h->n;
+    a.px = h->s.px;
+    a.py = h->s.py;
+    a.pz = h->s.pz;
+    a.m = h->s.mass;
+    a.rad = h->s.radius;
+    a.act = h->s.active;
+    a.eps2 = eps * eps;
+    a.acc[0] = h->s.ax;
+    a.acc[1] = h->s.ay;
+    a.acc[2] = h->s.az;
+    a.vel[0] = h->s.vx;
+    a.vel[1] = h->s.vy;
+    a.vel[2] = h->s.vz;
+    a.err = h->scal->err;
+    return a;
+}
+
+int fp64_order(int flags) {
+    return (flags & NB_FLAG_ORDER_PAIRWISE) ? nb::kOrderPairwise
+           : (flags & NB_FLAG_ORDER_SIMD)   ? nb::kOrderSimd
+                                            : nb::kOrderParallel;
+}
+
 // Forces for the current device rows.  kick: fuse the first half kick and
 // the drift of a Verlet step into the bounding-box pass.  dn (Barnes-Hut
 // modes only): the rows are counted on the device (a captured collisional
@@ -276,21 +303,19 @@ int force_pipeline(nb_engine* h, int flags, double eps, bool kick, double dt,
     Scal* sc = h->scal;
     h->tree_current = false;
     record(h, 0);
-    nb::launch_kick_drift_bbox(h->st, n, h->s, kick, dt, sc->bbox_ord, &sc->n_active, sc->err,
-                               dn);
-    cudaMemsetAsync(sc->counters, 0, sizeof(sc->counters), h->st);
     h->ev_tree = false;
+    // the FP64 direct sum needs no bounding box, and checks the positions itself
+    if (mode != NB_MODE_DIRECT_FP64 || kick)
+        nb::launch_kick_drift_bbox(h->st, n, h->s, kick, dt, sc->bbox_ord, &sc->n_active,
+                                   sc->err, dn);
+    cudaMemsetAsync(sc->counters, 0, sizeof(sc->counters), h->st);
     const int* dna = dn ? &sc->n_active : nullptr;
     if (dn && mode != NB_MODE_BARNES_HUT)
         return fail(h, NB_ERR_INVALID_ARG, "device row counts need NB_MODE_BARNES_HUT");
     if (mode == NB_MODE_DIRECT_FP64) {
         record(h, 1);
         record(h, 2);
-        const int order = (flags & NB_FLAG_ORDER_PAIRWISE) ? nb::kOrderPairwise
-                          : (flags & NB_FLAG_ORDER_SIMD)   ? nb::kOrderSimd
-                                                           : nb::kOrderParallel;
-        nb::direct_fp64(h->st, n, h->s.px, h->s.py, h->s.pz, h->s.mass, h->s.radius,
-                        h->s.active, eps, shell, order, h->s.ax, h->s.ay, h->s.az);
+        NB_CUDA(h, nb::direct_fp64(h->st, fp64_args(h, eps), shell, fp64_order(flags), h->sms));
         record(h, 3);
         h->counters[NB_C_BODY_INTERACTIONS] = (int64_t)h->n_active * (h->n_active - 1);
         h->counters[NB_C_CELL_INTERACTIONS] = 0;
@@ -517,6 +542,7 @@ NB_API int32_t nb_create(int32_t capacity, int32_t device, nb_engine** out) {
     }
     nb::sort_init();
     nb::walk_init(h->sms, h->wcfg);
+    nb::direct_init();
     const size_t cap = (size_t)capacity;
     do {
         if ((r = alloc_state(h, h->s, capacity))) break;
@@ -946,6 +972,27 @@ int run_steps(nb_engine* h, int n_steps, double dt, double softening, int flags)
     if (collide && n_steps > 1 && (flags & NB_MODE_MASK) == NB_MODE_BARNES_HUT &&
         !(flags & NB_FLAG_LEARNED_MAC))
         return run_collide_graphs(h, n_steps, dt, softening, flags);
+    double sub[3];
+    const int ns = sub_steps(flags, dt, sub);
+    if (!collide && (flags & NB_MODE_MASK) == NB_MODE_DIRECT_FP64 && (n_steps > 1 || ns == 1)) {
+        // the force kernel closes each step and opens the next: one launch a
+        // step, positions alternating between the state's and the compaction
+        // target's arrays
+        double* const pos[2][3] = {{h->s.px, h->s.py, h->s.pz},
+                                   {h->s_alt.px, h->s_alt.py, h->s_alt.pz}};
+        h->tree_current = false;
+        h->ev_tree = false;
+        NB_CUDA(h, cudaMemsetAsync(h->scal->counters, 0, sizeof(h->scal->counters), h->st));
+        for (int k = 0; k < 3; k++) record(h, k);
+        NB_CUDA(h, nb::direct_fp64_steps(h->st, fp64_args(h, softening),
+                                         (flags & NB_FLAG_SHELL_THEOREM) != 0, fp64_order(flags),
+                                         h->sms, pos, sub, ns, n_steps * ns));
+        record(h, 3);
+        h->ev_valid = h->timing != 0 && n_steps == 1;
+        if ((r = check_device(h))) return r;
+        collect_counters(h);
+        return NB_OK;
+    }
     if (!collide && n_steps > 1) {
         // Multi-step calls replay one captured step (a CUDA graph) n times;
         // the row and active counts do not change without collisions.
@@ -956,8 +1003,6 @@ int run_steps(nb_engine* h, int n_steps, double dt, double softening, int flags)
         collect_counters(h);
         return NB_OK;
     }
-    double sub[3];
-    const int ns = sub_steps(flags, dt, sub);
     for (int k = 0; k < n_steps * ns; k++) {
         const double sdt = sub[k % ns];
         if ((r = force_pipeline(h, flags, softening, true, sdt))) return r;
