@@ -17,6 +17,20 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return y;
 }
 
+// 1/sqrt(x) in FP64 from the hardware's approximation on the high word
+// (rsqrt.approx.ftz.f64: relative error at most 2^-20.0 over 2^32 arguments
+// spread over [1, 4)) and one third-order Householder step,
+// y <- y (1 + e/2 + 3e^2/8) with e = 1 - x y^2, which cubes the relative error
+// (2^-58 before FP64 rounding).  x = 0, subnormal, infinite or NaN takes
+// the library routine.
+__device__ __forceinline__ double rsqrt_f64(double x) {
+    if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) return rsqrt(x);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
 // Packed pairs of FP32 values (sm_100 f32x2 arithmetic): one instruction
 // applies the same IEEE-rounded operation to both halves.
 using f32x2 = unsigned long long;

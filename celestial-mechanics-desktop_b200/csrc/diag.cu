@@ -75,20 +75,6 @@ k_diag_final(int nblocks, const double* __restrict__ part, int n_items,
     }
 }
 
-// 1/sqrt(x) in FP64 from the hardware's approximation on the high word
-// (rsqrt.approx.ftz.f64: relative error at most 2^-20.0 over 2^32 arguments
-// spread over [1, 4)) and one third-order Householder step,
-// y <- y (1 + e/2 + 3e^2/8) with e = 1 - x y^2, which cubes the relative error
-// (2^-58 before FP64 rounding).  x = 0, subnormal, infinite or NaN takes
-// the library routine.
-__device__ __forceinline__ double rsqrt_f64(double x) {
-    if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) return rsqrt(x);
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // Exact pair potential, sum over active pairs i < j of
 // -m_i m_j / sqrt(r^2 + eps^2), as a grid of (tile of 512 rows, chunk of
 // sources) items that lie on or above the diagonal: each thread holds two

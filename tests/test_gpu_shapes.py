@@ -6,7 +6,9 @@ import numpy as np
 import pytest
 
 from conftest import bodies_dict
-from nbody_b200 import MODE_DIRECT_FP64, scenarios
+from helpers import rel_err
+from nbody_b200 import MODE_BARNES_HUT_REF, MODE_DIRECT_FP64, scenarios
+from nbody_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +42,46 @@ def test_fp64_direct_at_dispatch_edges(engine, oracle, n):
         v = oracle.verlet_direct(bodies_dict(b), 1e-4, 1e-3, steps)
         for k in ("px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az"):
             np.testing.assert_array_equal(getattr(s, k), v[k], err_msg=k)
+
+
+def _nested_corner(levels=9):
+    """A cell whose corner octant is subdivided again and again, every other
+    octant of each level holding one body in each of its own octants: a walk
+    that opens everything leaves 56 nodes behind on each level."""
+    pts = [(0.0005,) * 3, (0.9995,) * 3]
+    for lev in range(levels):
+        for o in range(1, 8):
+            for q in range(8):
+                pts.append(tuple(2.0 ** -(lev + 1) * (((o >> a) & 1) + 0.25 + 0.5 * ((q >> a) & 1))
+                                 for a in range(3)))
+    p = np.array(pts) * 2.002 - 1.001  # the octree's cube of a [-1, 1] box
+    n = len(p)
+    b = scenarios.plummer(n, seed=7)
+    b.px, b.py, b.pz = (np.ascontiguousarray(p[:, k]) for k in range(3))
+    b.mass = 1.0 + np.arange(n) % 5
+    return b
+
+
+@pytest.mark.parametrize("scene", [1, 2, 3, 4, 5, 31, 33, 1000, "corner", "disk"])
+def test_reference_walk_at_group_edges(engine, oracle, scene):
+    """The four-body warps of the reference walk, its narrow rounds when the
+    stack fills (the nested corner) and its shell leaves, against the oracle's
+    walk: the same cells, so FP64 rounding apart (the mode's 1e-9)."""
+    shell, theta = scene == "disk", 0.2 if scene == "corner" else 0.5
+    if shell:
+        b = scenarios.collisional_disk(601, seed=9, radius_scale=3000.0)
+    else:
+        b = _nested_corner() if scene == "corner" else scenarios.plummer(scene, seed=scene)
+    if b.n > 4:
+        b.active[4::13] = 0
+    want = oracle.bh_forces(b.px, b.py, b.pz, b.mass, b.active, 1e-4, theta, radius=b.radius,
+                            shell=shell)
+    engine.set_param(N.PARAM_THETA, theta)
+    got = engine.compute_forces(b.px, b.py, b.pz, b.mass, b.active, 1e-4,
+                                MODE_BARNES_HUT_REF | (N.FLAG_SHELL_THEOREM if shell else 0),
+                                radius=b.radius)
+    engine.set_param(N.PARAM_THETA, 0.5)
+    if b.n == 1:
+        assert got[0][0] == got[1][0] == got[2][0] == 0.0
+        return
+    assert rel_err(got, want)[b.active == 1].max() < 1e-9
