@@ -258,11 +258,71 @@ NB_WALK_EVAL void parts_two(const float* pbuf, int npair, float bx, float by, fl
     b = make_float3(fold2(UX), fold2(UY), fold2(UZ));
 }
 
-template <bool QUAD, bool SHELL, bool POT, bool GUARD, int MAC, int SHAPE = 0, int GS = 32>
+// Terms of the body list entries rep, rep + nrep, ... < np on one body, a
+// source of radius R pulling as a softened shell inside it (p1: R^2 and the
+// coefficient there).
+template <bool GUARD>
+NB_WALK_EVAL float3 parts_shell(const float* pbuf, const float2* p1, int np, int rep, int nrep,
+                                float bx, float by, float bz, float eps2) {
+    float tx = 0.f, ty = 0.f, tz = 0.f;
+#pragma unroll 4
+    for (int j = rep; j < np; j += nrep) {
+        const float* e = pbuf + (j >> 1) * 8 + (j & 1);
+        const float dx = bx - e[0], dy = by - e[2], dz = bz - e[4], pm = -e[6];
+        const float raw = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        const float r2 = raw + eps2;
+        const float inv = (GUARD && !(r2 > 0.f)) ? 0.f : rsqrt_ftz(r2);
+        float f = pm * (inv * inv * inv);
+        const float2 S = p1[j];
+        if (raw < S.x) f = S.y;
+        tx = fmaf(-f, dx, tx);
+        ty = fmaf(-f, dy, ty);
+        tz = fmaf(-f, dz, tz);
+    }
+    return make_float3(tx, ty, tz);
+}
+
+// Helping (HELP): a warp that finds no group left evaluates lists for the
+// warps of its block that still walk.  Groups differ: in a sparse outskirt 64
+// consecutive bodies span so large a box that their list holds nearly every
+// body, and a warp alone with such a list kept its SM at a quarter of its
+// issue slots while the others had ended.  A walking warp that has a list to
+// evaluate hands it to an idle warp of its block, takes that warp's empty list
+// buffer for it, and walks on; the helper leaves the lanes' FP32 sums in the
+// list's buffer, and the owner folds them into its compensated accumulators
+// in list order, so the forces are the same bits whoever evaluates.  While
+// every warp has a group of its own the cost is one shared-memory read per
+// list.  A warp that waits polls with pauses: waiting on an mbarrier instead
+// woke it so late that 50,000 bodies took 470 us, not 340 (plain: 600).
+constexpr int kHelpPolls = 1 << 22;  // bound of every wait between the warps of a block
+struct WalkHelp {
+    int idle;              // bit w: warp w waits for a list
+    int active;            // warps that still walk
+    int posted[kWalkWarps];  // a list waits for / is evaluated by warp w
+    int done[kWalkWarps];    // its sums are in the list's buffer
+    int owner[kWalkWarps];
+    int shape[kWalkWarps];   // entries | lw << 12 | two << 16 | particles << 17
+    int cells[kWalkWarps];   // warp w's cell / body buffer (offset in floats)
+    int parts[kWalkWarps];
+};
+__device__ __forceinline__ int ld_shared_volatile(const int* p) { return *(const volatile int*)p; }
+
+template <bool QUAD, bool SHELL, bool POT, bool GUARD, int MAC, int SHAPE = 0, int GS = 32,
+          bool HELP = false>
 __global__ void __launch_bounds__(WalkShape<MAC, SHAPE, GS>::warps * 32,
                                   WalkShape<MAC, SHAPE, GS>::min_blocks)
 k_walk_group(WalkArgs a) {
     constexpr int WARPS = WalkShape<MAC, SHAPE, GS>::warps;
+    static_assert(!HELP || (MAC == kMacGeometric && !POT), "helping walks");
+    __shared__ WalkHelp s_help;
+    if (HELP) {
+        if (threadIdx.x < WARPS) s_help.posted[threadIdx.x] = s_help.done[threadIdx.x] = 0;
+        if (threadIdx.x == 0) {
+            s_help.idle = 0;
+            s_help.active = WARPS;
+        }
+        __syncthreads();
+    }
     // two-body lanes evaluate each list block for both bodies in one pass
     // (one shared-memory read of the block for the two; each body's terms
     // are summed in the same order as in a pass per body).  The harvest walk
@@ -273,16 +333,22 @@ k_walk_group(WalkArgs a) {
     extern __shared__ __align__(16) float s_walk[];
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* base = s_walk + warp * kWarpFloats;
     // Interaction lists in a pair-blocked layout: field f of entry e sits at
     // [(e / 2) * W + 2 f + e % 2], so one 16-byte load returns two fields of
     // entries 2m and 2m+1 as register pairs for the packed f32x2 arithmetic.
     // cells (W = 20): rel x, y, z, -mass, Qxx, Qyy, Qzz, Qxy, Qxz, Qyz
     // bodies (W = 8): rel x, y, z, -mass
-    float* cbuf = base;
-    float* pbuf = base + kCellCap * 10;
+    float* const wbase = s_walk + warp * kWarpFloats;
+    float* cbuf = wbase;
+    float* pbuf = wbase + kCellCap * 10;
     float2* p1 = (float2*)(pbuf + kPartCap * 4);     // R^2, m / (R^2 + eps^2)^1.5
-    int* p2 = (int*)(p1 + kPartCap);                 // sorted index
+    int* p2 = (int*)(p1 + kPartCap);                 // sorted index (potential walks)
+    int coff = warp * kWarpFloats, poff = coff + kCellCap * 10;  // offsets of cbuf, pbuf (HELP)
+    // the lanes' bodies, for the helpers: in words that the variant has no
+    // other use for (the shell's buffers change hands with their lists)
+    constexpr int kPosOff = kCellCap * 10 + kPartCap * (SHELL ? 6 : 4);
+    static_assert(!HELP || (SHELL ? kPartCap : 3 * kPartCap) >= (GS == 64 ? 192 : 96), "positions");
+    float* const pos = wbase + kPosOff;
     int* fa = a.front + (size_t)(blockIdx.x * WARPS + warp) * a.front_cap;
     const float eps2 = (float)a.eps2;
     const float theta2 = (float)a.theta2;
@@ -300,10 +366,20 @@ k_walk_group(WalkArgs a) {
         pend = (int*)(ys + 32);
     }
 
+    // With helpers the first group of every warp is dealt out, one warp of each
+    // block after the other, so that few groups spread over all SMs (taken from
+    // the counter they go to whole blocks); the rest are taken as warps come free.
+    bool dealt = !HELP;
     for (;;) {
         int g = 0;
-        if (lane == 0) g = (int)atomicAdd(a.group_ctr, 1u);
-        g = __shfl_sync(FULL, g, 0);
+        if (HELP && !dealt) {
+            g = warp * (int)gridDim.x + (int)blockIdx.x;
+            dealt = true;
+        } else {
+            if (lane == 0) g = (int)atomicAdd(a.group_ctr, 1u);
+            g = __shfl_sync(FULL, g, 0);
+            if (HELP) g += WARPS * (int)gridDim.x;
+        }
         if (g >= ngroups) break;
         const int2 grp = a.groups[g];  // body_first, body_count (<= 64)
         const int nvalid = grp.y;
@@ -382,6 +458,116 @@ k_walk_group(WalkArgs a) {
         float spot2 = 0.f, cpot2 = 0.f;
         int nc = 0, np = 0;
         unsigned long long grp_entries = 0;  // list entries of this group (load-balance record)
+        // lists out with helpers, oldest first: 4 bits each, warp | particles << 3
+        unsigned out_fifo = 0;
+        int n_out = 0;
+        // lists are handed out once so few groups are left that warps may come
+        // free before this one ends
+        bool can_help = HELP && g + 4 * WARPS * (int)gridDim.x >= ngroups;
+        if (HELP) {
+            pos[lane] = bx;
+            pos[32 + lane] = by;
+            pos[64 + lane] = bz;
+            if (GS == 64) {
+                pos[96 + lane] = bx2;
+                pos[128 + lane] = by2;
+                pos[160 + lane] = bz2;
+            }
+        }
+        // Folds the oldest list that is out; wait: until its helper is done.
+        auto fold_one = [&](bool wait) -> bool {
+            const int w = out_fifo & 7;
+            int ok = 0;
+            if (lane == 0) {
+                for (int polls = 0; !(ok = ld_shared_volatile(&s_help.done[w])) && wait; polls++) {
+                    if (polls > kHelpPolls) break;
+                    __nanosleep(20);
+                }
+                if (!ok && wait) dev_flag(a.err, kErrTimeout);
+            }
+            ok = __shfl_sync(FULL, ok, 0);
+            if (!ok && !wait) return false;
+            __threadfence_block();
+            if (ok) {
+                const float* t = s_walk + ((out_fifo & 8) ? ld_shared_volatile(&s_help.parts[w])
+                                                          : ld_shared_volatile(&s_help.cells[w]));
+                kahan(sax, cax, t[lane]);
+                kahan(say, cay, t[32 + lane]);
+                kahan(saz, caz, t[64 + lane]);
+                if (GS == 64 && two) {
+                    kahan(sbx, cbx, t[96 + lane]);
+                    kahan(sby, cby, t[128 + lane]);
+                    kahan(sbz, cbz, t[160 + lane]);
+                }
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) {
+                    *(volatile int*)&s_help.done[w] = 0;
+                    __threadfence_block();
+                    atomicOr(&s_help.idle, 1 << w);
+                }
+            } else {
+                can_help = false;  // the launch has failed: nothing more is handed out
+            }
+            out_fifo >>= 4;
+            n_out--;
+            return true;
+        };
+        // Folds every list that is out.
+        auto fold_all = [&]() {
+            if constexpr (HELP) {
+                while (n_out > 0) fold_one(true);
+            }
+        };
+        // Hands a list of `entries` to an idle warp, if there is one.
+        auto hand_out = [&](int entries, bool parts) -> bool {
+            if constexpr (!HELP) {
+                return false;
+            } else {
+                while (n_out > 0 && fold_one(false)) {}
+                if (!can_help) return false;
+                int w = -1;
+                if (lane == 0) {
+                    int m = ld_shared_volatile(&s_help.idle);
+                    while (m) {
+                        const int bit = m & -m;
+                        const int old = atomicAnd(&s_help.idle, ~bit);
+                        if (old & bit) {
+                            w = __ffs(bit) - 1;
+                            break;
+                        }
+                        m = old & ~bit;
+                    }
+                }
+                w = __shfl_sync(FULL, w, 0);
+                if (w < 0) return false;
+                __threadfence_block();
+                int* theirs = parts ? &s_help.parts[w] : &s_help.cells[w];
+                const int spare = ld_shared_volatile(theirs);
+                __syncwarp();
+                if (lane == 0) {
+                    *(volatile int*)theirs = parts ? poff : coff;
+                    *(volatile int*)&s_help.owner[w] = warp;
+                    *(volatile int*)&s_help.shape[w] =
+                        entries | (lw << 12) | ((int)two << 16) | ((int)parts << 17);
+                    __threadfence_block();
+                    *(volatile int*)&s_help.posted[w] = 1;
+                }
+                __syncwarp();
+                if (parts) {
+                    poff = spare;
+                    pbuf = s_walk + poff;
+                    p1 = (float2*)(pbuf + kPartCap * 4);
+                } else {
+                    coff = spare;
+                    cbuf = s_walk + coff;
+                }
+                // at most WARPS - 1 lists are out, 4 bits each
+                out_fifo |= (unsigned)(w | ((int)parts << 3)) << (4 * n_out);
+                n_out++;
+                return true;
+            }
+        };
 
         // The cell list's terms on the body at (bx, by, bz) (group-centred).
         // Both bodies of a two-body lane in one pass over the cell list: each
@@ -442,15 +628,23 @@ k_walk_group(WalkArgs a) {
                     __syncwarp();
                 }
             }
+            if (hand_out(nc, false)) {
+                cnt_cell += (unsigned long long)nc * nvalid;
+                grp_entries += nc;
+                nc = 0;
+                return;
+            }
             float tx, ty, tz, tp;
             if (!POT && FUSE2 && two) {
                 float ux, uy, uz;
                 eval_cells2(tx, ty, tz, ux, uy, uz);
+                fold_all();
                 kahan(sbx, cbx, ux);
                 kahan(sby, cby, uy);
                 kahan(sbz, cbz, uz);
             } else {
                 eval_cells(bx, by, bz, tx, ty, tz, tp);
+                fold_all();
                 if (two) {
                     float ux, uy, uz, up;
                     eval_cells(bx2, by2, bz2, ux, uy, uz, up);
@@ -479,8 +673,10 @@ k_walk_group(WalkArgs a) {
         auto eval_parts = [&](float bx, float by, float bz, int self, float& tx, float& ty,
                               float& tz, float& tp) {
             tx = ty = tz = tp = 0.f;
-            if constexpr (!SHELL && !POT) {
-                const float3 t3 = parts_one<GUARD>(pbuf, (np + 1) >> 1, rep, nrep, bx, by, bz, eps2);
+            if constexpr (!POT) {
+                const float3 t3 =
+                    SHELL ? parts_shell<GUARD>(pbuf, p1, np, rep, nrep, bx, by, bz, eps2)
+                          : parts_one<GUARD>(pbuf, (np + 1) >> 1, rep, nrep, bx, by, bz, eps2);
                 tx = t3.x;
                 ty = t3.y;
                 tz = t3.z;
@@ -514,15 +710,23 @@ k_walk_group(WalkArgs a) {
                     __syncwarp();
                 }
             }
+            if (hand_out(np, true)) {
+                cnt_body += (unsigned long long)np * nvalid;
+                grp_entries += np;
+                np = 0;
+                return;
+            }
             float tx, ty, tz, tp;
             if (!SHELL && !POT && FUSE2 && two) {
                 float ux, uy, uz;
                 eval_parts2(tx, ty, tz, ux, uy, uz);
+                fold_all();
                 kahan(sbx, cbx, ux);
                 kahan(sby, cby, uy);
                 kahan(sbz, cbz, uz);
             } else {
                 eval_parts(bx, by, bz, s, tx, ty, tz, tp);
+                fold_all();
                 if (two) {
                     float ux, uy, uz, up;
                     eval_parts(bx2, by2, bz2, s2, ux, uy, uz, up);
@@ -809,6 +1013,7 @@ k_walk_group(WalkArgs a) {
         }
         if (nc) flush_cells();
         if (np) flush_parts();
+        fold_all();
         if (lane == 0 && a.counters) atomicMax(&a.counters[2], grp_entries);
         // combine the replicas of each body (lanes equal modulo the width)
         double fx = (double)sax - (double)cax, fy = (double)say - (double)cay;
@@ -838,6 +1043,74 @@ k_walk_group(WalkArgs a) {
         atomicAdd(&a.counters[0], cnt_cell);
         atomicAdd(&a.counters[1], cnt_body);
         if (MAC == kMacLearned) atomicAdd(&a.counters[3], cnt_mlp);
+    }
+    if constexpr (HELP) {
+        // no group left: evaluate the others' lists until they have ended too
+        if (lane == 0) {
+            *(volatile int*)&s_help.cells[warp] = coff;
+            *(volatile int*)&s_help.parts[warp] = poff;
+            __threadfence_block();
+            atomicOr(&s_help.idle, 1 << warp);
+            atomicSub(&s_help.active, 1);
+        }
+        for (int polls = 0;;) {
+            int job = 0;  // 1 a list, 2 leave
+            if (lane == 0) {
+                if (ld_shared_volatile(&s_help.posted[warp])) {
+                    job = 1;
+                } else if (ld_shared_volatile(&s_help.active) == 0) {
+                    job = 2;
+                } else if (++polls > kHelpPolls) {
+                    // waited long enough: leave unless a list is on its way
+                    if (atomicAnd(&s_help.idle, ~(1 << warp)) & (1 << warp)) job = 2;
+                }
+            }
+            job = __shfl_sync(FULL, job, 0);
+            if (job == 2) break;
+            if (job == 0) {
+                __nanosleep(100);
+                continue;
+            }
+            __threadfence_block();
+            const int shape = ld_shared_volatile(&s_help.shape[warp]);
+            const float* q = s_walk + ld_shared_volatile(&s_help.owner[warp]) * kWarpFloats + kPosOff;
+            const int entries = shape & 0xFFF, lw = (shape >> 12) & 0xF;
+            const int rep = lane >> lw, nrep = 32 >> lw;
+            const bool parts = (shape >> 17) & 1;
+            float* list = s_walk + ld_shared_volatile(parts ? &s_help.parts[warp] : &s_help.cells[warp]);
+            const int npair = (entries + 1) >> 1;
+            const float hx = q[lane], hy = q[32 + lane], hz = q[64 + lane];
+            float3 t, u = make_float3(0.f, 0.f, 0.f);
+            if (GS == 64 && ((shape >> 16) & 1)) {
+                const float ix = q[96 + lane], iy = q[128 + lane], iz = q[160 + lane];
+                if (parts) parts_two<GUARD>(list, npair, hx, hy, hz, ix, iy, iz, eps2, t, u);
+                else cells_two<QUAD>(list, npair, hx, hy, hz, ix, iy, iz, eps2, t, u);
+            } else if (!parts) {
+                t = cells_one<QUAD>(list, npair, rep, nrep, hx, hy, hz, eps2);
+            } else if (SHELL) {
+                t = parts_shell<GUARD>(list, (const float2*)(list + kPartCap * 4), entries, rep, nrep,
+                                       hx, hy, hz, eps2);
+            } else {
+                t = parts_one<GUARD>(list, npair, rep, nrep, hx, hy, hz, eps2);
+            }
+            __syncwarp();  // the whole list is read before the sums overwrite it
+            list[lane] = t.x;
+            list[32 + lane] = t.y;
+            list[64 + lane] = t.z;
+            if (GS == 64) {
+                list[96 + lane] = u.x;
+                list[128 + lane] = u.y;
+                list[160 + lane] = u.z;
+            }
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) {
+                *(volatile int*)&s_help.posted[warp] = 0;
+                __threadfence_block();
+                *(volatile int*)&s_help.done[warp] = 1;
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -1101,30 +1374,41 @@ void find_groups(cudaStream_t st, const TreeBufs& t, const double4* sbody, int n
 
 using WalkKernel = void (*)(WalkArgs);
 
-// The instantiated variants: (quad) x {plain, shell, potential} x (guard).
-static WalkKernel pick_walk(bool quad, bool shell, bool pot, bool guard) {
-#define NB_WALK_PICK(Q, S, P)                                            \
-    return guard ? k_walk_group<Q, S, P, true, kMacGeometric>                \
-                 : k_walk_group<Q, S, P, false, kMacGeometric>
-    if (pot) {
-        if (quad) NB_WALK_PICK(true, false, true);
-        NB_WALK_PICK(false, false, true);
-    }
-    if (shell) {
-        if (quad) NB_WALK_PICK(true, true, false);
-        NB_WALK_PICK(false, true, false);
-    }
-    if (quad) NB_WALK_PICK(true, false, false);
-    NB_WALK_PICK(false, false, false);
-#undef NB_WALK_PICK
+// The instantiated variants: (quad) x {plain, shell, potential} x (guard) x
+// (helping; not the potential's).
+template <bool QUAD, bool GUARD, bool HELP>
+static WalkKernel pick_walk(bool shell, bool pot) {
+    if (pot) return k_walk_group<QUAD, false, true, GUARD, kMacGeometric>;
+    if (shell) return k_walk_group<QUAD, true, false, GUARD, kMacGeometric, 0, 32, HELP>;
+    return k_walk_group<QUAD, false, false, GUARD, kMacGeometric, 0, 32, HELP>;
+}
+template <bool QUAD, bool GUARD>
+static WalkKernel pick_walk(bool shell, bool pot, bool help) {
+    return help ? pick_walk<QUAD, GUARD, true>(shell, pot) : pick_walk<QUAD, GUARD, false>(shell, pot);
+}
+static WalkKernel pick_walk(bool quad, bool shell, bool pot, bool guard, bool help) {
+    if (quad)
+        return guard ? pick_walk<true, true>(shell, pot, help) : pick_walk<true, false>(shell, pot, help);
+    return guard ? pick_walk<false, true>(shell, pot, help) : pick_walk<false, false>(shell, pot, help);
+}
+// 64-body groups, geometric
+static WalkKernel pick_walk64(bool guard, bool help) {
+    if (help)
+        return guard ? k_walk_group<true, false, false, true, kMacGeometric, 0, 64, true>
+                     : k_walk_group<true, false, false, false, kMacGeometric, 0, 64, true>;
+    return guard ? k_walk_group<true, false, false, true, kMacGeometric, 0, 64>
+                 : k_walk_group<true, false, false, false, kMacGeometric, 0, 64>;
 }
 
 void walk_init(int sms, WalkConfig& cfg) {
-    for (int v = 0; v < 16; v++) {
+    for (int v = 0; v < 32; v++) {
         const bool pot = v & 4, shell = (v & 2) && !pot;
-        cudaFuncSetAttribute((const void*)pick_walk(v & 1, shell, pot, v & 8),
+        cudaFuncSetAttribute((const void*)pick_walk(v & 1, shell, pot, v & 8, v & 16),
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
     }
+    for (int v = 0; v < 4; v++)
+        cudaFuncSetAttribute((const void*)pick_walk64(v & 1, v & 2),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem64);
     cudaFuncSetAttribute((const void*)k_walk_group<true, false, false, false, kMacHarvest>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
     cudaFuncSetAttribute((const void*)k_walk_group<true, false, false, false, kMacLearned>,
@@ -1159,13 +1443,10 @@ void walk_init(int sms, WalkConfig& cfg) {
     if (cfg.blocks_small * kWalkWarpsSmall > cfg.blocks * kWalkWarps)
         cfg.blocks_small = cfg.blocks * kWalkWarps / kWalkWarpsSmall;
     // the 64-body-group variants
-    const void* g64[4] = {(const void*)k_walk_group<true, false, false, false, kMacGeometric, 0, 64>,
-                          (const void*)k_walk_group<true, false, false, true, kMacGeometric, 0, 64>,
-                          (const void*)k_walk_group<true, false, false, false, kMacHarvest, 0, 64>,
-                          (const void*)k_walk_group<true, false, false, false, kMacLearned, 0, 64>};
-    for (int k = 0; k < 4; k++)
-        cudaFuncSetAttribute(g64[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             k == 3 ? kWalkSmemMac64 : kWalkSmem64);
+    cudaFuncSetAttribute((const void*)k_walk_group<true, false, false, false, kMacHarvest, 0, 64>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem64);
+    cudaFuncSetAttribute((const void*)k_walk_group<true, false, false, false, kMacLearned, 0, 64>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmemMac64);
     int per_sm64 = 0, per_sm_mac64 = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm64, k_walk_group<true, false, false, false, kMacGeometric, 0, 64>,
@@ -1194,6 +1475,12 @@ void walk_group(cudaStream_t st, const WalkConfig& cfg, WalkArgs a, bool quad, b
     // quadrupole walks without the shell theorem or potentials
     const bool g64 = a.group_size == 64 && a.group_span >= 64 && quad && !shell && !pot &&
                      (mac != kMacGeometric || shape == 0);
+    // Helping pays while the grid's warps have at most some three groups each:
+    // plain -> helping at theta 0.5, 64-body groups, 20,011 bodies 455 -> 207 us,
+    // 100,003 730 -> 590, 400,000 2,080 -> 2,020; 2^20 (seven groups per warp)
+    // 5,370 -> 5,420, and 576,000 bodies in 137 systems lose 2 %.  The forces are
+    // the same bits either way.
+    auto help_pays = [&](int warps, int size) { return a.n <= 3LL * warps * size; };
     find_groups(st, a.t, a.sbody, a.n, a.groups, a.n_groups, a.pack, a.group_span,
                 g64 ? 64 : 32);
     cudaMemsetAsync(a.group_ctr, 0, sizeof(unsigned), st);
@@ -1204,11 +1491,8 @@ void walk_group(cudaStream_t st, const WalkConfig& cfg, WalkArgs a, bool quad, b
         else if (mac == kMacLearned)
             k_walk_group<true, false, false, false, kMacLearned, 0, 64>
                 <<<cfg.blocks_mac64, kMacWarps64 * 32, kWalkSmemMac64, st>>>(a);
-        else if (a.eps2 > 0.0)
-            k_walk_group<true, false, false, false, kMacGeometric, 0, 64>
-                <<<cfg.blocks64, NB_WALK64_WARPS * 32, kWalkSmem64, st>>>(a);
         else
-            k_walk_group<true, false, false, true, kMacGeometric, 0, 64>
+            pick_walk64(!(a.eps2 > 0.0), help_pays(cfg.blocks64 * NB_WALK64_WARPS, 64))
                 <<<cfg.blocks64, NB_WALK64_WARPS * 32, kWalkSmem64, st>>>(a);
         return;
     }
@@ -1229,7 +1513,7 @@ void walk_group(cudaStream_t st, const WalkConfig& cfg, WalkArgs a, bool quad, b
         k<<<cfg.blocks_small, kWalkWarpsSmall * 32, kWalkWarpsSmall * kWarpFloats * 4, st>>>(a);
         return;
     }
-    const WalkKernel k = pick_walk(quad, shell, pot, !(a.eps2 > 0.0));
+    const WalkKernel k = pick_walk(quad, shell, pot, !(a.eps2 > 0.0), help_pays(cfg.blocks * kWalkWarps, 32));
     k<<<cfg.blocks, kWalkThreads, kWalkSmem, st>>>(a);
 }
 

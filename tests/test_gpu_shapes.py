@@ -7,7 +7,7 @@ import pytest
 
 from conftest import bodies_dict
 from helpers import rel_err
-from nbody_b200 import MODE_BARNES_HUT_REF, MODE_DIRECT_FP64, scenarios
+from nbody_b200 import MODE_BARNES_HUT, MODE_BARNES_HUT_REF, MODE_DIRECT_FP64, scenarios
 from nbody_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
@@ -85,3 +85,33 @@ def test_reference_walk_at_group_edges(engine, oracle, scene):
         assert got[0][0] == got[1][0] == got[2][0] == 0.0
         return
     assert rel_err(got, want)[b.active == 1].max() < 1e-9
+
+
+@pytest.mark.parametrize("shell", [False, True])
+@pytest.mark.parametrize("eps", [0.0, 1e-4])
+@pytest.mark.parametrize("n", [1, 33, 65, 1000, 20011, 500000])
+def test_group_walk_helping_range(engine, oracle, n, eps, shell):
+    """The walk with and without helping warps (n on both sides of the rule),
+    64- and 32-body groups, with zero softening too: the sampled bodies within
+    the mode's 1e-3 rms of the FP64 direct sum, the counts of a second call the
+    same and its forces the same bits."""
+    b = scenarios.plummer(n, seed=n)
+    b.radius[:] = 1e-3
+    flags = MODE_BARNES_HUT | (N.FLAG_SHELL_THEOREM if shell else 0)
+    engine.set_param(N.PARAM_THETA, 0.5)
+
+    def forces():
+        f = engine.compute_forces(b.px, b.py, b.pz, b.mass, b.active, eps, flags, radius=b.radius)
+        return np.array(f), engine.counters()[:2].tolist()
+
+    got, counts = forces()
+    again, counts2 = forces()
+    np.testing.assert_array_equal(got, again)
+    assert counts == counts2
+    t = np.unique(np.linspace(0, n - 1, min(n, 256)).astype(np.int32))
+    want = np.array(oracle.direct_forces_targets(b.px, b.py, b.pz, b.mass, b.active, eps, t,
+                                                 radius=b.radius, shell=shell))
+    den = np.sqrt((want ** 2).sum(0))
+    err = np.sqrt(((got[:, t] - want) ** 2).sum(0))[den > 0] / den[den > 0]
+    assert np.isfinite(got).all()
+    assert err.size == 0 or np.sqrt(np.mean(err ** 2)) < 1e-3
