@@ -20,6 +20,7 @@
 #include "collide.cuh"
 #include "diag.cuh"
 #include "direct.cuh"
+#include "hostio.cuh"
 #include "sort.cuh"
 #include "tree.cuh"
 #include "walk.cuh"
@@ -138,6 +139,9 @@ struct nb_engine {
     nb::CollideBufs col{};
     Scal* scal = nullptr;
     std::vector<void*> allocs;
+    nb::HostIO io;                        // copies to and from the caller's arrays
+    Scal* scal_host = nullptr;            // pinned: the scalars as of the last check, and
+    int* nodes_host = nullptr;            // the node count
     // timing
     cudaEvent_t ev[6] = {};
     // captured single step (CUDA graph) and the parameters it was captured with
@@ -210,30 +214,65 @@ int dalloc(nb_engine* h, T** p, size_t count) {
 
 int alloc_state(nb_engine* h, nb::State& s, int cap) {
     int r = NB_OK;
-    double** d[] = {&s.px, &s.py, &s.pz, &s.vx, &s.vy, &s.vz, &s.ax, &s.ay, &s.az,
-                    &s.mass, &s.radius, &s.density};
-    for (double** p : d)
-        if ((r = dalloc(h, p, cap))) return r;
+    // one block, rows evenly spaced: the rows of one call travel as one 2-D copy
+    double** d[] = {&s.mass, &s.px, &s.py, &s.pz, &s.vx, &s.vy, &s.vz, &s.ax, &s.ay, &s.az,
+                    &s.radius, &s.density};
+    const size_t pitch = ((size_t)cap + 31) / 32 * 32;
+    double* block = nullptr;
+    if ((r = dalloc(h, &block, pitch * (sizeof(d) / sizeof(d[0]))))) return r;
+    for (double** p : d) {
+        *p = block;
+        block += pitch;
+    }
     if ((r = dalloc(h, &s.active, cap))) return r;
     if ((r = dalloc(h, &s.collidable, cap))) return r;
     return dalloc(h, &s.ids, cap);
 }
 
-// Collect the device error word and the last CUDA error after a sync.
+// Synchronise, and collect the device's error words, its other scalars (into
+// scal_host) and the last CUDA error.
 int check_device(nb_engine* h) {
-    cudaError_t e = cudaStreamSynchronize(h->st);
+    cudaError_t e = cudaMemcpyAsync(h->scal_host, h->scal, sizeof(Scal), cudaMemcpyDeviceToHost, h->st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(h->nodes_host, h->tree.n_nodes, sizeof(int), cudaMemcpyDeviceToHost, h->st);
+    if (e != cudaSuccess) return fail(h, NB_ERR_CUDA, "error word: %s", cudaGetErrorString(e));
+    e = cudaStreamSynchronize(h->st);
     if (e != cudaSuccess) return fail(h, NB_ERR_CUDA, "stream: %s", cudaGetErrorString(e));
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(h, NB_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
-    int err[nb::kErrCount];
-    e = cudaMemcpy(err, h->scal->err, sizeof(err), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return fail(h, NB_ERR_CUDA, "error word: %s", cudaGetErrorString(e));
-    cudaMemsetAsync(h->scal->err, 0, sizeof(err), h->st);
+    const int* err = h->scal_host->err;
+    bool any = false;
+    for (int k = 0; k < nb::kErrCount; k++) any = any || err[k];
+    if (!any) return NB_OK;
+    cudaMemsetAsync(h->scal->err, 0, sizeof(h->scal->err), h->st);
     if (err[nb::kErrNonFinite]) return fail(h, NB_ERR_NONFINITE, "non-finite position or mass");
     if (err[nb::kErrTimeout]) return fail(h, NB_ERR_TIMEOUT, "a bounded device wait expired");
     if (err[nb::kErrOverflow])
         return fail(h, NB_ERR_STACK_OVERFLOW, "tree-walk frontier overflow");
-    if (err[nb::kErrCapacity]) return fail(h, NB_ERR_CAPACITY, "device buffer capacity exceeded");
+    return fail(h, NB_ERR_CAPACITY, "device buffer capacity exceeded");
+}
+
+// Arrays of one transfer; null or empty ones are left out.
+struct Segs {
+    nb::CopySeg seg[16];
+    int n = 0;
+    void add(void* dst, const void* src, size_t bytes) {
+        if (dst && src && bytes) seg[n++] = {dst, src, bytes};
+    }
+};
+
+int send(nb_engine* h, const Segs& s) {
+    NB_CUDA(h, nb::copy_up(h->io, h->st, s.seg, s.n));
+    return NB_OK;
+}
+
+// Waits for the stream, checks the device and brings the arrays to the host.
+int receive(nb_engine* h, const Segs& s) {
+    bool queued = false;
+    int r;
+    NB_CUDA(h, nb::start_down(h->io, h->st, s.seg, s.n, &queued));
+    if ((r = check_device(h))) return r;
+    NB_CUDA(h, nb::finish_down(h->io, h->st, s.seg, s.n, queued));
     return NB_OK;
 }
 
@@ -463,21 +502,23 @@ int step_graph(nb_engine* h, int flags, double dt, double eps) {
     return NB_OK;
 }
 
+// Counters of the last evaluation, from the scalars of the last check.
 void collect_counters(nb_engine* h) {
-    unsigned long long c[4];
-    if (cudaMemcpy(c, h->scal->counters, sizeof(c), cudaMemcpyDeviceToHost) == cudaSuccess) {
-        h->counters[NB_C_CELL_INTERACTIONS] = (int64_t)c[0];
-        h->counters[NB_C_BODY_INTERACTIONS] = (int64_t)c[1];
-        h->counters[NB_C_MAX_GROUP_WORK] = (int64_t)c[2];
-        h->counters[NB_C_MAC_EVALS] = (int64_t)c[3];
+    const unsigned long long* c = h->scal_host->counters;
+    h->counters[NB_C_CELL_INTERACTIONS] = (int64_t)c[0];
+    h->counters[NB_C_BODY_INTERACTIONS] = (int64_t)c[1];
+    h->counters[NB_C_MAX_GROUP_WORK] = (int64_t)c[2];
+    h->counters[NB_C_MAC_EVALS] = (int64_t)c[3];
+    if (h->ev_tree) {
+        h->counters[NB_C_NODES] = *h->nodes_host;
+        h->counters[NB_C_GROUPS] = h->scal_host->n_groups;
     }
-    int nn = 0;
-    if (h->ev_tree && cudaMemcpy(&nn, h->tree.n_nodes, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess)
-        h->counters[NB_C_NODES] = nn;
-    int ng = 0;
-    if (h->ev_tree && cudaMemcpy(&ng, &h->scal->n_groups, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess)
-        h->counters[NB_C_GROUPS] = ng;
     h->counters[NB_C_ACTIVE] = h->n_active;
+}
+
+__global__ void k_row_ids(int n, int32_t* __restrict__ ids) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) ids[i] = i;
 }
 
 int count_active_host(const uint8_t* a, int n) {
@@ -487,27 +528,28 @@ int count_active_host(const uint8_t* a, int n) {
 }
 
 // Upload positions / masses / radii / active into the device rows (the
-// host-array entry points stage through the state arrays).
+// host-array entry points stage through the state arrays).  `more` arrays
+// travel with them.  A null mass or radius array leaves zeros.
 int stage_bodies(nb_engine* h, int n, const double* px, const double* py, const double* pz,
-                 const double* mass, const double* radius, const uint8_t* active) {
+                 const double* mass, const double* radius, const uint8_t* active,
+                 const Segs* more = nullptr) {
     int r;
     if ((r = check_n(h, n))) return r;
     if (n > 0 && (!px || !py || !pz || !active))
         return fail(h, NB_ERR_INVALID_ARG, "null position or active array");
     const size_t d = sizeof(double) * (size_t)n;
-    if ((r = upload(h, h->s.px, px, d)) || (r = upload(h, h->s.py, py, d)) ||
-        (r = upload(h, h->s.pz, pz, d)) || (r = upload(h, h->s.active, active, (size_t)n)))
-        return r;
-    if (mass) {
-        if ((r = upload(h, h->s.mass, mass, d))) return r;
-    } else {
-        NB_CUDA(h, cudaMemsetAsync(h->s.mass, 0, d, h->st));
-    }
-    if (radius) {
-        if ((r = upload(h, h->s.radius, radius, d))) return r;
-    } else {
-        NB_CUDA(h, cudaMemsetAsync(h->s.radius, 0, d, h->st));
-    }
+    Segs s;
+    s.add(h->s.mass, mass, d);
+    s.add(h->s.px, px, d);
+    s.add(h->s.py, py, d);
+    s.add(h->s.pz, pz, d);
+    if (more)
+        for (int k = 0; k < more->n; k++) s.seg[s.n++] = more->seg[k];
+    s.add(h->s.radius, radius, d);
+    s.add(h->s.active, active, (size_t)n);
+    if ((r = send(h, s))) return r;
+    if (!mass) NB_CUDA(h, cudaMemsetAsync(h->s.mass, 0, d, h->st));
+    if (!radius) NB_CUDA(h, cudaMemsetAsync(h->s.radius, 0, d, h->st));
     h->n = n;
     h->n_active = n > 0 ? count_active_host(active, n) : 0;
     h->has_state = false;
@@ -575,6 +617,13 @@ NB_API int32_t nb_create(int32_t capacity, int32_t device, nb_engine** out) {
              })))
             break;
         if ((r = dalloc(h, &h->scal, 1))) break;
+        // a call's arrays up to 256 KB go through the handle's own pinned memory
+        nb::hostio_init(h->io, device, std::min<size_t>(1 << 18, 128 * cap + 8192));
+        if (cudaHostAlloc((void**)&h->scal_host, sizeof(Scal) + 64, cudaHostAllocDefault) != cudaSuccess) {
+            r = fail(h, NB_ERR_CUDA, "pinned scalars");
+            break;
+        }
+        h->nodes_host = (int*)(h->scal_host + 1);
         if (cudaMemset(h->scal, 0, sizeof(Scal)) != cudaSuccess) { r = NB_ERR_CUDA; break; }
         for (auto& e : h->ev)
             if (cudaEventCreate(&e) != cudaSuccess) { r = NB_ERR_CUDA; break; }
@@ -592,6 +641,8 @@ NB_API int32_t nb_destroy(nb_engine* h) {
     cudaSetDevice(h->device);
     if (h->st) cudaStreamSynchronize(h->st);
     for (void* p : h->allocs) cudaFree(p);
+    nb::hostio_free(h->io);
+    if (h->scal_host) cudaFreeHost(h->scal_host);
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
     if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
@@ -746,14 +797,18 @@ NB_API int32_t nb_compute_forces(nb_engine* h, int32_t n, const double* px, cons
     if (!mass && n > 0) return fail(h, NB_ERR_INVALID_ARG, "null mass array");
     if (n > 0 && (!ax || !ay || !az)) return fail(h, NB_ERR_INVALID_ARG, "null output array");
     int r;
-    if ((r = stage_bodies(h, n, px, py, pz, mass, radius, active))) return r;
+    // only the shell theorem reads radii here
+    if ((r = stage_bodies(h, n, px, py, pz, mass,
+                          (flags & NB_FLAG_SHELL_THEOREM) ? radius : nullptr, active)))
+        return r;
     if (n == 0) return NB_OK;
     if ((r = force_pipeline(h, flags, softening, false, 0.0))) return r;
     const size_t d = sizeof(double) * (size_t)n;
-    if ((r = download(h, ax, h->s.ax, d)) || (r = download(h, ay, h->s.ay, d)) ||
-        (r = download(h, az, h->s.az, d)))
-        return r;
-    if ((r = check_device(h))) return r;
+    Segs s;
+    s.add(ax, h->s.ax, d);
+    s.add(ay, h->s.ay, d);
+    s.add(az, h->s.az, d);
+    if ((r = receive(h, s))) return r;
     collect_counters(h);
     return NB_OK;
 }
@@ -768,33 +823,26 @@ NB_API int32_t nb_set_state(nb_engine* h, int32_t n, const double* px, const dou
     int r;
     if (n > 0 && (!vx || !vy || !vz || !mass))
         return fail(h, NB_ERR_INVALID_ARG, "null velocity or mass array");
-    if ((r = stage_bodies(h, n, px, py, pz, mass, radius, active))) return r;
-    const size_t d = sizeof(double) * (size_t)n;
-    if ((r = upload(h, h->s.vx, vx, d)) || (r = upload(h, h->s.vy, vy, d)) ||
-        (r = upload(h, h->s.vz, vz, d)))
-        return r;
+    const size_t d = n > 0 ? sizeof(double) * (size_t)n : 0;
+    Segs more;
+    if (n >= 0 && n <= h->capacity) {
+        more.add(h->s.vx, vx, d);
+        more.add(h->s.vy, vy, d);
+        more.add(h->s.vz, vz, d);
+        more.add(h->s.ax, oax, d);
+        more.add(h->s.ay, oay, d);
+        more.add(h->s.az, oaz, d);
+        more.add(h->s.density, density, d);
+        more.add(h->s.collidable, collidable, (size_t)n);
+    }
+    if ((r = stage_bodies(h, n, px, py, pz, mass, radius, active, &more))) return r;
     double* acc[3] = {h->s.ax, h->s.ay, h->s.az};
     const double* old[3] = {oax, oay, oaz};
-    for (int k = 0; k < 3; k++) {
-        if (old[k]) {
-            if ((r = upload(h, acc[k], old[k], d))) return r;
-        } else {
-            NB_CUDA(h, cudaMemsetAsync(acc[k], 0, d, h->st));
-        }
-    }
-    if (density) {
-        if ((r = upload(h, h->s.density, density, d))) return r;
-    } else {
-        NB_CUDA(h, cudaMemsetAsync(h->s.density, 0, d, h->st));
-    }
-    if (collidable) {
-        if ((r = upload(h, h->s.collidable, collidable, (size_t)n))) return r;
-    } else {
-        NB_CUDA(h, cudaMemsetAsync(h->s.collidable, 1, (size_t)n, h->st));
-    }
-    std::vector<int32_t> ids((size_t)n);
-    for (int i = 0; i < n; i++) ids[i] = i;
-    if ((r = upload(h, h->s.ids, ids.data(), sizeof(int32_t) * (size_t)n))) return r;
+    for (int k = 0; k < 3; k++)
+        if (!old[k]) NB_CUDA(h, cudaMemsetAsync(acc[k], 0, d, h->st));
+    if (!density) NB_CUDA(h, cudaMemsetAsync(h->s.density, 0, d, h->st));
+    if (!collidable) NB_CUDA(h, cudaMemsetAsync(h->s.collidable, 1, (size_t)n, h->st));
+    if (n > 0) k_row_ids<<<nb::ceil_div(n, 256), 256, 0, h->st>>>(n, h->s.ids);
     if ((r = check_device(h))) return r;
     h->has_state = true;
     h->adapt_dt = 0.0;
@@ -811,17 +859,21 @@ NB_API int32_t nb_get_state(nb_engine* h, int32_t* n_out, double* px, double* py
     const int n = h->n;
     if (n_out) *n_out = n;
     const size_t d = sizeof(double) * (size_t)n;
-    int r;
-    if ((r = download(h, px, h->s.px, d)) || (r = download(h, py, h->s.py, d)) ||
-        (r = download(h, pz, h->s.pz, d)) || (r = download(h, vx, h->s.vx, d)) ||
-        (r = download(h, vy, h->s.vy, d)) || (r = download(h, vz, h->s.vz, d)) ||
-        (r = download(h, ax, h->s.ax, d)) || (r = download(h, ay, h->s.ay, d)) ||
-        (r = download(h, az, h->s.az, d)) || (r = download(h, mass, h->s.mass, d)) ||
-        (r = download(h, radius, h->s.radius, d)) ||
-        (r = download(h, active, h->s.active, (size_t)n)) ||
-        (r = download(h, ids, h->s.ids, sizeof(int32_t) * (size_t)n)))
-        return r;
-    return check_device(h);
+    Segs s;
+    s.add(mass, h->s.mass, d);
+    s.add(px, h->s.px, d);
+    s.add(py, h->s.py, d);
+    s.add(pz, h->s.pz, d);
+    s.add(vx, h->s.vx, d);
+    s.add(vy, h->s.vy, d);
+    s.add(vz, h->s.vz, d);
+    s.add(ax, h->s.ax, d);
+    s.add(ay, h->s.ay, d);
+    s.add(az, h->s.az, d);
+    s.add(radius, h->s.radius, d);
+    s.add(active, h->s.active, (size_t)n);
+    s.add(ids, h->s.ids, sizeof(int32_t) * (size_t)n);
+    return receive(h, s);
 }
 
 namespace {
@@ -953,13 +1005,11 @@ int run_collide_graphs(nb_engine* h, int n_steps, double dt, double eps, int fla
     h->tree_current = false;
     h->ev_valid = false;
     h->ev_collide = false;
-    int cnt[4] = {0, 0, 0, 0};  // n_pairs, n_kept, n_merges, n_rows
-    if ((r = download(h, cnt, &h->scal->n_pairs, sizeof(cnt)))) return r;
-    r = check_device(h);  // synchronises: cnt holds the last step's counts
-    h->n = cnt[3];
-    h->n_active = cnt[3];  // compaction keeps exactly the active rows
-    h->counters[NB_C_PAIRS] = cnt[0];
-    h->counters[NB_C_MERGES] = cnt[2];
+    r = check_device(h);  // synchronises: the scalars hold the last step's counts
+    h->n = h->scal_host->n_rows;
+    h->n_active = h->n;  // compaction keeps exactly the active rows
+    h->counters[NB_C_PAIRS] = h->scal_host->n_pairs;
+    h->counters[NB_C_MERGES] = h->scal_host->n_merges;
     if (r) return r;
     collect_counters(h);
     return NB_OK;

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "bodies.cuh"
+#include "hostio.cuh"
 #include "sort.cuh"
 #include "tree.cuh"
 #include "walk.cuh"
@@ -364,12 +365,27 @@ __global__ void k_ens_energy(int n, const int* __restrict__ sys_of_all, const in
     }
 }
 
-__global__ void k_permute(int n, const int* __restrict__ perm, const double* __restrict__ src,
-                          double* __restrict__ dst, int scatter) {
+// Up to nine fields between the caller's row order and the handle's: gather
+// (dst[k][i] = src[k][perm[i]], a non-finite value sets the error word) or
+// scatter (dst[k][perm[i]] = src[k][i]).
+struct PermuteArgs {
+    const double* src[9];
+    double* dst[9];
+    int fields;
+};
+__global__ void k_permute(int n, const int* __restrict__ perm, PermuteArgs f, int scatter, int* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (scatter) dst[perm[i]] = src[i];
-    else dst[i] = src[perm[i]];
+    const int p = perm[i];
+    for (int k = 0; k < f.fields; k++) {
+        if (scatter) {
+            f.dst[k][p] = f.src[k][i];
+        } else {
+            const double v = f.src[k][p];
+            if (!isfinite(v)) dev_flag(err, kErrNonFinite);
+            f.dst[k][i] = v;
+        }
+    }
 }
 
 }  // namespace
@@ -400,7 +416,8 @@ struct nb_ensemble {
     nb::State s{}, sbh{};
     int *d_off = nullptr, *d_off_bh = nullptr, *d_sys_of_bh = nullptr, *d_sys_of = nullptr;
     int* d_perm = nullptr;                // internal row -> caller row
-    double* d_stage = nullptr;
+    double* d_stage = nullptr;            // nine rows of n: fields in the caller's order
+    nb::HostIO io;                        // copies to and from the caller's arrays
     double4* d_cubes = nullptr;           // per system (internal order)
     double* d_half16 = nullptr;
     double4* d_com = nullptr;
@@ -736,7 +753,7 @@ NB_API int32_t nb_ens_create(int32_t n_systems, const int32_t* sizes, int32_t ds
         if ((r = ealloc(h, &h->d_off, (size_t)n_systems + 1))) break;
         if ((r = ealloc(h, &h->d_off_bh, (size_t)h->nbh + 1))) break;
         if ((r = ealloc(h, &h->d_sys_of, n)) || (r = ealloc(h, &h->d_sys_of_bh, nbhb))) break;
-        if ((r = ealloc(h, &h->d_perm, n)) || (r = ealloc(h, &h->d_stage, n))) break;
+        if ((r = ealloc(h, &h->d_perm, n)) || (r = ealloc(h, &h->d_stage, 9 * n))) break;
         if ((r = ealloc(h, &h->d_cubes, (size_t)n_systems)) ||
             (r = ealloc(h, &h->d_half16, (size_t)n_systems)) ||
             (r = ealloc(h, &h->d_com, (size_t)n_systems)) ||
@@ -798,6 +815,7 @@ NB_API int32_t nb_ens_create(int32_t n_systems, const int32_t* sizes, int32_t ds
         nb_ens_destroy(h);
         return r;
     }
+    nb::hostio_init(h->io, device, std::min<size_t>(1 << 18, 80 * n + 8192));
     *out = h;
     return NB_OK;
 }
@@ -809,6 +827,7 @@ NB_API int32_t nb_ens_destroy(nb_ensemble* h) {
     if (h->st2) cudaStreamSynchronize(h->st2);
     if (h->graph) cudaGraphExecDestroy(h->graph);
     for (void* p : h->allocs) cudaFree(p);
+    nb::hostio_free(h->io);
     for (cudaEvent_t e : {h->ev_fork, h->ev_join, h->ev_t0, h->ev_t1})
         if (e) cudaEventDestroy(e);
     if (h->st2) cudaStreamDestroy(h->st2);
@@ -883,20 +902,25 @@ NB_API int32_t nb_ens_set_state(nb_ensemble* h, const double* px, const double* 
     cudaSetDevice(h->device);
     const double* src[] = {px, py, pz, vx, vy, vz, mass};
     double* dst[] = {h->s.px, h->s.py, h->s.pz, h->s.vx, h->s.vy, h->s.vz, h->s.mass};
+    const size_t n = (size_t)h->n;
+    nb::CopySeg seg[7];
+    nb::PermuteArgs f{};
+    f.fields = 7;
     for (int k = 0; k < 7; k++) {
-        for (size_t i = 0; i < (size_t)h->n; i++)
-            if (!std::isfinite(src[k][i])) return efail(h, NB_ERR_NONFINITE, "non-finite input");
-        NE_CUDA(h, cudaMemcpyAsync(h->d_stage, src[k], sizeof(double) * h->n,
-                                   cudaMemcpyHostToDevice, h->st));
-        nb::k_permute<<<nb::ceil_div(h->n, 256), 256, 0, h->st>>>(h->n, h->d_perm, h->d_stage,
-                                                                 dst[k], 0);
+        seg[k] = {h->d_stage + k * n, src[k], sizeof(double) * n};
+        f.src[k] = h->d_stage + k * n;
+        f.dst[k] = dst[k];
     }
+    NE_CUDA(h, nb::copy_up(h->io, h->st, seg, 7));
+    nb::k_permute<<<nb::ceil_div(h->n, 256), 256, 0, h->st>>>(h->n, h->d_perm, f, 0, h->scal->err);
     NE_CUDA(h, cudaMemsetAsync(h->s.ax, 0, sizeof(double) * h->n, h->st));
     NE_CUDA(h, cudaMemsetAsync(h->s.ay, 0, sizeof(double) * h->n, h->st));
     NE_CUDA(h, cudaMemsetAsync(h->s.az, 0, sizeof(double) * h->n, h->st));
+    const int r = ens_check(h);
+    if (r) return r;
     h->has_state = true;
     h->has_acc = false;
-    return ens_check(h);
+    return NB_OK;
 }
 
 NB_API int32_t nb_ens_get_state(nb_ensemble* h, double* px, double* py, double* pz, double* vx,
@@ -907,15 +931,24 @@ NB_API int32_t nb_ens_get_state(nb_ensemble* h, double* px, double* py, double* 
     double* dst[] = {px, py, pz, vx, vy, vz, ax, ay, az};
     const double* src[] = {h->s.px, h->s.py, h->s.pz, h->s.vx, h->s.vy, h->s.vz,
                            h->s.ax, h->s.ay, h->s.az};
+    const size_t n = (size_t)h->n;
+    nb::CopySeg seg[9];
+    nb::PermuteArgs f{};
     for (int k = 0; k < 9; k++) {
         if (!dst[k]) continue;
-        nb::k_permute<<<nb::ceil_div(h->n, 256), 256, 0, h->st>>>(h->n, h->d_perm, src[k],
-                                                                 h->d_stage, 1);
-        NE_CUDA(h, cudaMemcpyAsync(dst[k], h->d_stage, sizeof(double) * h->n,
-                                   cudaMemcpyDeviceToHost, h->st));
-        NE_CUDA(h, cudaStreamSynchronize(h->st));
+        double* row = h->d_stage + f.fields * n;
+        seg[f.fields] = {dst[k], row, sizeof(double) * n};
+        f.src[f.fields] = src[k];
+        f.dst[f.fields++] = row;
     }
-    return ens_check(h);
+    if (f.fields > 0)
+        nb::k_permute<<<nb::ceil_div(h->n, 256), 256, 0, h->st>>>(h->n, h->d_perm, f, 1, h->scal->err);
+    bool queued = false;
+    NE_CUDA(h, nb::start_down(h->io, h->st, seg, f.fields, &queued));
+    const int r = ens_check(h);
+    if (r) return r;
+    NE_CUDA(h, nb::finish_down(h->io, h->st, seg, f.fields, queued));
+    return NB_OK;
 }
 
 NB_API int32_t nb_ens_compute_forces(nb_ensemble* h, double softening) {

@@ -1,0 +1,42 @@
+// hostio.cuh - copies between the caller's pageable arrays and the device.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+namespace nb {
+
+// One array of a transfer; `dst` / `src` is host or device memory by direction.
+struct CopySeg {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+
+struct CopyPool;
+
+// A handle's side of the transfers: a pinned buffer of its own for small ones
+// (two halves, up and down, so a call may fill one while the other is read)
+// and its share of the device's copy pool for large ones.
+struct HostIO {
+    char* pin = nullptr;
+    size_t half = 0;
+    int device = 0;
+    CopyPool* pool = nullptr;
+};
+
+// io is usable (with slower copies) even when this fails.
+void hostio_init(HostIO& io, int device, size_t half_bytes);
+void hostio_free(HostIO& io);
+
+// Host arrays to the device in stream order.  On return the host arrays may
+// be changed.  An earlier upload through the same handle has to have ended.
+cudaError_t copy_up(HostIO& io, cudaStream_t st, const CopySeg* seg, int n);
+
+// Device arrays to the host.  start_down enqueues what fits the pinned half
+// (adjacent rows in one copy) and reports in *queued whether everything did;
+// after the stream has been synchronised finish_down puts the data into the
+// host arrays, by the pool where start_down queued nothing.
+cudaError_t start_down(HostIO& io, cudaStream_t st, const CopySeg* seg, int n, bool* queued);
+cudaError_t finish_down(HostIO& io, cudaStream_t st, const CopySeg* seg, int n, bool queued);
+
+}  // namespace nb

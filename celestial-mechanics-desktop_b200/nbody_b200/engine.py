@@ -25,6 +25,14 @@ class NBodyError(RuntimeError):
         self.status = status
 
 
+_VECTORS = ("px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az")
+
+
+def _writable_f64(a, n: int) -> bool:
+    return (isinstance(a, np.ndarray) and a.dtype == np.float64 and a.shape == (n,)
+            and a.flags.c_contiguous and a.flags.aligned and a.flags.writeable)
+
+
 class Engine:
     """One engine handle: a CUDA stream and device buffers for `capacity` bodies."""
 
@@ -114,19 +122,35 @@ class Engine:
                                        N.ptr(rad), N.ptr(dens), N.ptr(act), N.ptr(col),
                                        *(N.ptr(a) for a in acc)))
 
+    def body_count(self) -> int:
+        """Rows of the device state."""
+        n, active = np.zeros(1, np.int32), np.zeros(1, np.int32)
+        self._check(N.lib.nb_get_body_count(self._h, N.ptr(n), N.ptr(active)))
+        return int(n[0])
+
     def get_state(self) -> tuple[Bodies, np.ndarray]:
         n_out = np.zeros(1, np.int32)
-        cap = self.capacity
-        f = {k: np.empty(cap) for k in ("px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az",
-                                         "mass", "radius")}
-        act = np.empty(cap, np.uint8)
-        ids = np.empty(cap, np.int32)
-        self._check(N.lib.nb_get_state(self._h, N.ptr(n_out), *(N.ptr(f[k]) for k in (
-            "px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az", "mass", "radius")),
-            N.ptr(act), N.ptr(ids)))
-        n = int(n_out[0])
-        b = Bodies(**{k: v[:n].copy() for k, v in f.items()}, active=act[:n].copy())
-        return b, ids[:n].copy()
+        n = self.body_count()
+        f = {k: np.empty(n) for k in (*_VECTORS, "mass", "radius")}
+        act = np.empty(n, np.uint8)
+        ids = np.empty(n, np.int32)
+        self._check(N.lib.nb_get_state(self._h, N.ptr(n_out), *(N.ptr(f[k]) for k in f),
+                                       N.ptr(act), N.ptr(ids)))
+        return Bodies(**f, active=act), ids
+
+    def get_vectors(self, b: Bodies):
+        """Positions, velocities and accelerations into the arrays of `b`,
+        which holds as many rows as the device."""
+        if b.n != self.body_count():
+            raise ValueError("the bodies do not match the device state")
+        got = {k: getattr(b, k) for k in _VECTORS}
+        # straight into arrays the engine can write, by way of others elsewhere
+        to = {k: a if _writable_f64(a, b.n) else np.empty(b.n) for k, a in got.items()}
+        self._check(N.lib.nb_get_state(self._h, None, *(N.ptr(to[k]) for k in _VECTORS), None,
+                                       None, None, None))
+        for k, a in got.items():
+            if to[k] is not a:
+                a[:] = to[k]
 
     def step(self, n_steps: int, dt: float, softening: float, flags: int):
         self._check(N.lib.nb_step(self._h, int(n_steps), float(dt), float(softening), int(flags)))
@@ -339,6 +363,4 @@ class B200SoAIntegrator:
         e.set_param(N.PARAM_THETA, float(backend.theta))
         e.set_state(bodies)
         e.step(n_steps, dt, softening, backend.flags())
-        out, _ = e.get_state()
-        for k in ("px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az"):
-            getattr(bodies, k)[:] = getattr(out, k)
+        e.get_vectors(bodies)

@@ -115,3 +115,41 @@ def test_group_walk_helping_range(engine, oracle, n, eps, shell):
     err = np.sqrt(((got[:, t] - want) ** 2).sum(0))[den > 0] / den[den > 0]
     assert np.isfinite(got).all()
     assert err.size == 0 or np.sqrt(np.mean(err ** 2)) < 1e-3
+
+
+@pytest.mark.parametrize("n", [1, 1000, 2016, 2017, 6001, 30000, 300001])
+def test_state_round_trip_at_transfer_sizes(engine, n):
+    """Host arrays below and above the pinned half and the pool's chunks, rows
+    that are views, and flags: every array comes back bit for bit."""
+    rng = np.random.default_rng(n)
+    b = scenarios.plummer(n, seed=n)
+    for k in ("px", "vy", "az", "radius"):
+        setattr(b, k, rng.standard_normal(2 * n)[::2])  # not contiguous
+    for k in ("ax", "ay"):
+        setattr(b, k, rng.standard_normal(n))
+    b.active = rng.integers(0, 2, n).astype(np.uint8)
+    engine.set_state(b)
+    s, ids = engine.get_state()
+    for k in ("px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az", "mass", "radius", "active"):
+        np.testing.assert_array_equal(getattr(s, k), getattr(b, k), err_msg=k)
+    np.testing.assert_array_equal(ids, np.arange(n))
+
+
+def test_transfers_of_two_threads():
+    """Two handles in two threads share the copy pool: each gets its own data."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from nbody_b200 import Engine
+
+    def one(seed):
+        b = scenarios.plummer(200_000 + seed, seed=seed)
+        with Engine(b.n) as e:
+            for _ in range(6):
+                e.set_state(b)
+                s, _ = e.get_state()
+                for k in ("px", "vz", "mass"):
+                    np.testing.assert_array_equal(getattr(s, k), getattr(b, k))
+        return True
+
+    with ThreadPoolExecutor(2) as ex:
+        assert all(ex.map(one, (1, 2)))
