@@ -18,22 +18,39 @@ struct State {
 // Every launcher's optional `dn` is a device row count that replaces n when
 // smaller (the grid stays sized for n): a captured step whose rows shrink
 // after each compaction reads its current row count there.
-// bbox_ord: 6 order-mapped words (min xyz, max xyz), reset to (~0, 0)
-// before the kernel.  n_active: active count (reset to 0).
+// Where the bounding-box pass puts the box of the active rows (6 order-mapped
+// words: min xyz, max xyz; ~0 and 0 when there is none), their count, and the
+// cube (cx, cy, cz, half) around them (gpu_tree.cu:163-167).  part: scratch of
+// box_part_bytes(); ticket: a word that is 0 between launches.
+struct BoxBufs {
+    unsigned long long* ord;
+    int* n_active;
+    double* cube;
+    double* part;
+    unsigned* ticket;
+};
+size_t box_part_bytes();
+// Words that the bounding-box pass zeroes for the kernels behind it.
+struct ZeroWords {
+    uint32_t* range = nullptr;  // e.g. the sort's workspace
+    size_t words = 0;
+    int* w[12] = {};            // single words (null: none)
+};
 void launch_kick_drift_bbox(cudaStream_t st, int n, State s, bool kick, double dt,
-                            unsigned long long* bbox_ord, int* n_active, int* err,
+                            const BoxBufs& box, const ZeroWords& zero, int* err,
                             const int* dn = nullptr);
+// The kick and drift alone (and the check for non-finite values).
+void launch_kick_drift(cudaStream_t st, int n, State s, double dt, int* err);
 void launch_kick(cudaStream_t st, int n, State s, double dt, const int* dn = nullptr);
-// Cube (cx, cy, cz, half) from the bbox words (gpu_tree.cu:163-167), or a
-// given cube when `given` is non-null.
-void launch_cube(cudaStream_t st, const unsigned long long* bbox_ord, const double* given,
-                 double* cube);
-// Octree-aligned keys in the cube + all 8 digit histograms (hist zeroed).
+// A cube given by the caller.
+void launch_cube(cudaStream_t st, const double* given, double* cube);
+// Octree-aligned keys in the cube + all 8 digit histograms (hist zeroed before).
 // Optionally, by row: rows = (x, y, z, m) and amag = |acc| (the previous
-// step's acceleration), for launch_gather.
+// step's acceleration), for launch_gather.  zero_acc: the accelerations of
+// inactive rows become 0 (the force kernels write the active ones).
 void launch_keys_cube(cudaStream_t st, int n, const State& s, const double* cube,
                       uint64_t* keys, uint32_t* vals, uint32_t* hist, double4* rows = nullptr,
-                      float* amag = nullptr, const int* dn = nullptr);
+                      float* amag = nullptr, bool zero_acc = false, const int* dn = nullptr);
 // Reference keys: per-axis AABB, scale 2^21-1 (morton_kernel.cu:11-76).
 void launch_keys_aabb(cudaStream_t st, int n, const State& s,
                       const unsigned long long* bbox_ord, uint64_t* keys, uint32_t* vals);
@@ -45,7 +62,4 @@ void launch_gather(cudaStream_t st, int n, const State& s, const uint32_t* sidx,
                    double4* sbody, float* srad, float* samag = nullptr,
                    const double4* rows = nullptr, const float* amag = nullptr,
                    const int* dn = nullptr);
-// Zero acc of all rows (inactive rows keep 0).
-void launch_zero_acc(cudaStream_t st, int n, State s, const int* dn = nullptr);
-
 }  // namespace nb

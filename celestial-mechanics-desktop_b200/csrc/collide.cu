@@ -238,10 +238,13 @@ int broad_phase(cudaStream_t st, CollideBufs& b, CollideArgs& a, bool build_tree
     *np = 0;
     if (a.n <= 0) return NB_OK;
     if (!a.reuse_tree) {
-        if (build_tree) {
-            launch_kick_drift_bbox(st, a.n, a.s, false, 0.0, a.bbox_ord, a.n_active_dev, a.err);
-            launch_cube(st, a.bbox_ord, nullptr, a.cube);
-        }
+        ZeroWords zero;
+        zero.range = (uint32_t*)a.sort_ws;
+        zero.words = sort_zero_words(a.n, a.sms);
+        if (build_tree)
+            launch_kick_drift_bbox(st, a.n, a.s, false, 0.0, a.box, zero, a.err);
+        else
+            cudaMemsetAsync(a.sort_ws, 0, sizeof(uint32_t) * zero.words, st);
         launch_keys_cube(st, a.n, a.s, a.cube, a.keys0, a.vals0, (uint32_t*)a.sort_ws);
         sort_pairs(st, a.n, a.keys0, a.vals0, a.keys1, a.vals1, a.sort_ws, true, a.err, a.sms);
         launch_gather(st, a.n_active, a.s, a.vals0, a.sbody, a.srad);

@@ -37,8 +37,7 @@ struct CollideArgs {
     int *n_pairs, *n_kept, *n_merges;
     int* err;
     int sms;
-    unsigned long long* bbox_ord;
-    int* n_active_dev;
+    BoxBufs box;
     // the force evaluation of this step left a tree of the current positions
     // (keys0/vals0 sorted, sbody/srad gathered, multipole pass with radii,
     // cube): the broad phase queries it instead of building its own

@@ -48,6 +48,7 @@ struct Scal {
     int n_merges;
     int n_rows;  // current row count of a captured collisional step
     unsigned long long amax2;  // bits of the largest |a|^2 (adaptive dt)
+    unsigned box_ticket;       // blocks of the bounding-box pass that have ended
 };
 
 }  // namespace
@@ -130,6 +131,7 @@ struct nb_engine {
     int* front = nullptr;
     double* rows = nullptr;
     double* part = nullptr;
+    double* box_part = nullptr;           // the bounding-box pass's block results
     double* phi = nullptr;
     int32_t* targets = nullptr;
     int2* groups = nullptr;
@@ -299,6 +301,39 @@ void record(nb_engine* h, int k) {
     if (h->timing) cudaEventRecord(h->ev[k], h->st);
 }
 
+// The bounding-box pass's outputs; its cube goes to scal->cube.
+nb::BoxBufs box_bufs(nb_engine* h) {
+    return {h->scal->bbox_ord, &h->scal->n_active, h->scal->cube, h->box_part, &h->scal->box_ticket};
+}
+
+// The counting words of a sort of n pairs.
+nb::ZeroWords sort_words(nb_engine* h, int n) {
+    nb::ZeroWords z;
+    z.range = (uint32_t*)h->sort_ws;
+    z.words = nb::sort_zero_words(n, h->sms);
+    return z;
+}
+
+// ... and those of the tree and the walk behind it.
+nb::ZeroWords force_words(nb_engine* h, int n) {
+    nb::ZeroWords z = sort_words(h, n);
+    z.w[0] = &h->scal->n_groups;
+    z.w[1] = (int*)&h->scal->group_ctr;
+    for (int k = 0; k < 8; k++) z.w[2 + k] = (int*)h->scal->counters + k;
+    return z;
+}
+
+// Bounding cube of the staged rows, or the caller's (cube4), into scal->cube.
+int stage_cube(nb_engine* h, const double* cube4) {
+    int r;
+    nb::launch_kick_drift_bbox(h->st, h->n, h->s, false, 0.0, box_bufs(h), sort_words(h, h->n),
+                               h->scal->err);
+    if (!cube4) return NB_OK;
+    if ((r = upload(h, h->scal->cube_in, cube4, sizeof(double) * 4))) return r;
+    nb::launch_cube(h->st, h->scal->cube_in, h->scal->cube);
+    return NB_OK;
+}
+
 // The FP64 direct sum's arguments for the current device rows.
 nb::Fp64Args fp64_args(nb_engine* h, double eps) {
     nb::Fp64Args a{};
@@ -345,9 +380,10 @@ int force_pipeline(nb_engine* h, int flags, double eps, bool kick, double dt,
     h->ev_tree = false;
     // the FP64 direct sum needs no bounding box, and checks the positions itself
     if (mode != NB_MODE_DIRECT_FP64 || kick)
-        nb::launch_kick_drift_bbox(h->st, n, h->s, kick, dt, sc->bbox_ord, &sc->n_active,
+        nb::launch_kick_drift_bbox(h->st, n, h->s, kick, dt, box_bufs(h), force_words(h, n),
                                    sc->err, dn);
-    cudaMemsetAsync(sc->counters, 0, sizeof(sc->counters), h->st);
+    if (mode == NB_MODE_DIRECT_FP64)
+        cudaMemsetAsync(sc->counters, 0, sizeof(sc->counters), h->st);
     const int* dna = dn ? &sc->n_active : nullptr;
     if (dn && mode != NB_MODE_BARNES_HUT)
         return fail(h, NB_ERR_INVALID_ARG, "device row counts need NB_MODE_BARNES_HUT");
@@ -370,16 +406,15 @@ int force_pipeline(nb_engine* h, int flags, double eps, bool kick, double dt,
                     "theorem and softening > 0");
     if (learned && !h->mac_ready)
         return fail(h, NB_ERR_STATE, "the learned MAC has no trained parameters");
-    nb::launch_cube(h->st, sc->bbox_ord, nullptr, sc->cube);
     // the keys kernel also writes each row's (x, y, z, m) record and, for the
-    // learned MAC, the previous step's |a| (before the buffer is zeroed)
+    // learned MAC, the previous step's |a|, and zeroes inactive rows'
+    // accelerations (the force kernels write the others)
     nb::launch_keys_cube(h->st, n, h->s, sc->cube, h->keys0, h->vals0, (uint32_t*)h->sort_ws,
-                         h->rows4, learned ? h->amag_rows : nullptr, dn);
+                         h->rows4, learned ? h->amag_rows : nullptr, true, dn);
     nb::sort_pairs(h->st, n, h->keys0, h->vals0, h->keys1, h->vals1, h->sort_ws, true, sc->err,
                    h->sms, dn);
     nb::launch_gather(h->st, na, h->s, h->vals0, h->sbody, radii ? h->srad : nullptr,
                       learned ? h->samag : nullptr, h->rows4, h->amag_rows, dna);
-    nb::launch_zero_acc(h->st, n, h->s, dn);
     record(h, 1);
     if (mode == NB_MODE_DIRECT) {
         record(h, 2);
@@ -414,6 +449,7 @@ int force_pipeline(nb_engine* h, int flags, double eps, bool kick, double dt,
         a.group_span = h->group_span;
         a.group_size = h->group_bodies;
         a.counters = sc->counters;
+        a.zeroed = true;
         a.err = sc->err;
         if (ref) {
             const double te = h->theta < 0.2 ? 0.2 : h->theta;  // barnes_hut_solver.cpp:16
@@ -599,6 +635,7 @@ NB_API int32_t nb_create(int32_t capacity, int32_t device, nb_engine** out) {
         if ((r = dalloc(h, (char**)&h->front, nb::walk_front_bytes(h->wcfg)))) break;
         if ((r = dalloc(h, &h->rows, cap)) || (r = dalloc(h, &h->phi, cap))) break;
         if ((r = dalloc(h, (char**)&h->part, nb::diag_partial_bytes(capacity)))) break;
+        if ((r = dalloc(h, (char**)&h->box_part, nb::box_part_bytes()))) break;
         if ((r = dalloc(h, &h->targets, cap)) || (r = dalloc(h, &h->tgt_out, 3 * cap))) break;
         if ((r = dalloc(h, (char**)&h->tgt_part, nb::direct_targets_scratch_bytes(h->sms)))) break;
         if ((r = dalloc(h, (char**)&h->aud_part, nb::audit_targets_scratch_bytes(h->sms)))) break;
@@ -904,8 +941,7 @@ nb::CollideArgs collide_args(nb_engine* h) {
     c.n_merges = &h->scal->n_merges;
     c.err = h->scal->err;
     c.sms = h->sms;
-    c.bbox_ord = h->scal->bbox_ord;
-    c.n_active_dev = &h->scal->n_active;
+    c.box = box_bufs(h);
     // the second half kick moved no body: the force evaluation's tree
     // (Barnes-Hut modes) still describes the positions
     c.reuse_tree = h->tree_current;
@@ -1174,8 +1210,7 @@ NB_API int32_t nb_diagnostics(nb_engine* h, double softening, int32_t pe_mode, d
         // tree potential: a walk with the potential accumulated
         const int n = h->n;
         Scal* sc = h->scal;
-        nb::launch_kick_drift_bbox(h->st, n, h->s, false, 0.0, sc->bbox_ord, &sc->n_active, sc->err);
-        nb::launch_cube(h->st, sc->bbox_ord, nullptr, sc->cube);
+        if ((r = stage_cube(h, nullptr))) return r;
         nb::launch_keys_cube(h->st, n, h->s, sc->cube, h->keys0, h->vals0, (uint32_t*)h->sort_ws);
         nb::sort_pairs(h->st, n, h->keys0, h->vals0, h->keys1, h->vals1, h->sort_ws, true, sc->err, h->sms);
         nb::launch_gather(h->st, h->n_active, h->s, h->vals0, h->sbody, nullptr);
@@ -1366,12 +1401,10 @@ NB_API int32_t nb_morton_keys(nb_engine* h, int32_t n, const double* px, const d
     if ((r = stage_bodies(h, n, px, py, pz, nullptr, nullptr, active))) return r;
     if (n == 0) return NB_OK;
     Scal* sc = h->scal;
-    nb::launch_kick_drift_bbox(h->st, n, h->s, false, 0.0, sc->bbox_ord, &sc->n_active, sc->err);
+    if ((r = stage_cube(h, mode == 0 ? nullptr : cube4))) return r;
     if (mode == 0) {
         nb::launch_keys_aabb(h->st, n, h->s, sc->bbox_ord, h->keys0, h->vals0);
     } else {
-        if (cube4 && (r = upload(h, sc->cube_in, cube4, sizeof(double) * 4))) return r;
-        nb::launch_cube(h->st, sc->bbox_ord, cube4 ? sc->cube_in : nullptr, sc->cube);
         nb::launch_keys_cube(h->st, n, h->s, sc->cube, h->keys0, h->vals0, (uint32_t*)h->sort_ws);
         if ((r = download(h, cube4_out, sc->cube, sizeof(double) * 4))) return r;
     }
@@ -1415,9 +1448,7 @@ NB_API int32_t nb_build_octree(nb_engine* h, int32_t n, const double* px, const 
     *n_nodes = 0;
     if (n == 0) return NB_OK;
     Scal* sc = h->scal;
-    nb::launch_kick_drift_bbox(h->st, n, h->s, false, 0.0, sc->bbox_ord, &sc->n_active, sc->err);
-    if (cube4 && (r = upload(h, sc->cube_in, cube4, sizeof(double) * 4))) return r;
-    nb::launch_cube(h->st, sc->bbox_ord, cube4 ? sc->cube_in : nullptr, sc->cube);
+    if ((r = stage_cube(h, cube4))) return r;
     nb::launch_keys_cube(h->st, n, h->s, sc->cube, h->keys0, h->vals0, (uint32_t*)h->sort_ws);
     nb::sort_pairs(h->st, n, h->keys0, h->vals0, h->keys1, h->vals1, h->sort_ws, true, sc->err,
                    h->sms);
@@ -1524,8 +1555,7 @@ NB_API int32_t nb_broad_phase(nb_engine* h, int32_t n, const double* px, const d
     c.n_pairs = &sc->n_pairs;
     c.err = sc->err;
     c.sms = h->sms;
-    c.bbox_ord = sc->bbox_ord;
-    c.n_active_dev = &sc->n_active;
+    c.box = box_bufs(h);
     c.groups = h->groups;
     c.n_groups = &sc->n_groups;
     c.group_ctr = &sc->group_ctr;
@@ -1577,12 +1607,11 @@ NB_API int32_t nb_mac_harvest(nb_engine* h, int32_t max_records, double sample_f
     }
     const int n = h->n, na = h->n_active;
     Scal* sc = h->scal;
-    nb::launch_kick_drift_bbox(h->st, n, h->s, false, 0.0, sc->bbox_ord, &sc->n_active, sc->err);
-    nb::launch_cube(h->st, sc->bbox_ord, nullptr, sc->cube);
-    nb::launch_keys_cube(h->st, n, h->s, sc->cube, h->keys0, h->vals0, (uint32_t*)h->sort_ws);
+    if ((r = stage_cube(h, nullptr))) return r;
+    nb::launch_keys_cube(h->st, n, h->s, sc->cube, h->keys0, h->vals0, (uint32_t*)h->sort_ws,
+                         nullptr, nullptr, true);
     nb::sort_pairs(h->st, n, h->keys0, h->vals0, h->keys1, h->vals1, h->sort_ws, true, sc->err, h->sms);
     nb::launch_gather(h->st, na, h->s, h->vals0, h->sbody, nullptr, h->samag);
-    nb::launch_zero_acc(h->st, n, h->s);
     nb::tree_build(h->st, h->tree, na, h->keys0, h->sbody, nullptr, sc->cube, h->leaf_cap, sc->err);
     NB_CUDA(h, cudaMemsetAsync(h->mac_counts, 0, sizeof(int) * 4, h->st));
     nb::WalkArgs a{};

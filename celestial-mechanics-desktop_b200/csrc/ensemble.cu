@@ -39,8 +39,6 @@ namespace nb {
 namespace {
 
 struct EnsScal {
-    unsigned long long bbox_ord[6];
-    int n_active;
     unsigned group_ctr;
     int n_groups;
     unsigned ds_ctr;
@@ -556,7 +554,7 @@ void launch_tree(nb_ensemble* h, cudaStream_t st, double eps) {
         const double4* cubes = h->d_cubes + h->nds;  // tree systems follow the direct ones
         const double* half16 = h->d_half16 + h->nds;
         uint32_t* hist = (uint32_t*)h->sort_ws;
-        cudaMemsetAsync(hist, 0, sizeof(uint32_t) * 8 * 256, st);
+        cudaMemsetAsync(hist, 0, sizeof(uint32_t) * nb::sort_zero_words(n, h->sms), st);
         nb::k_ens_keys<<<nb::ceil_div(n, 256 * nb::kEnsKeyItems), 256, 0, st>>>(
             n, h->sbh, h->d_sys_of_bh, cubes, h->keys0, h->vals0, hist);
         nb::sort_pairs(st, n, h->keys0, h->vals0, h->keys1, h->vals1, h->sort_ws, true, sc->err,
@@ -650,7 +648,7 @@ int ens_graph(nb_ensemble* h, double dt, double eps) {
     }
     NE_CUDA(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
     EnsScal* sc = h->scal;
-    nb::launch_kick_drift_bbox(h->st, h->n, h->s, true, dt, sc->bbox_ord, &sc->n_active, sc->err);
+    nb::launch_kick_drift(h->st, h->n, h->s, dt, sc->err);
     enqueue_forces(h, eps);
     nb::launch_kick(h->st, h->n, h->s, dt);
     cudaGraph_t g = nullptr;

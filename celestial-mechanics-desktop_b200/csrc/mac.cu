@@ -215,6 +215,7 @@ void mac_adam(cudaStream_t st, float* P, const float* G, float* m, float* v, int
 // - log2 d and f1, f4 as in mac_features), and log2 of its mass.
 __global__ void k_mac_node_terms(TreeBufs t, const MacDev* __restrict__ w,
                                  float2* __restrict__ out) {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *t.n_nodes) return;
     const float mass = (float)t.com[i].w;
@@ -230,7 +231,7 @@ __global__ void k_mac_node_terms(TreeBufs t, const MacDev* __restrict__ w,
 }
 
 void mac_node_terms(cudaStream_t st, const TreeBufs& t, int n, const MacDev* w, float2* out) {
-    if (n > 0) k_mac_node_terms<<<ceil_div(2LL * n, 256), 256, 0, st>>>(t, w, out);
+    if (n > 0) launch_pdl(n, k_mac_node_terms, ceil_div(2LL * n, 256), 256, 0, st, t, w, out);
 }
 
 // ---- prediction (the walk's inference routine on given feature rows) -------

@@ -117,6 +117,7 @@ k_sort_pass(int n, int shift, const uint64_t* __restrict__ kin, const uint32_t* 
     constexpr int kSortItems = ITEMS;
     constexpr int kSortTile = kSortThreads * ITEMS;
     extern __shared__ __align__(16) unsigned char s_dyn[];
+    pdl_enter();
     uint64_t* s_keys = (uint64_t*)s_dyn;                    // tile-sorted keys
     uint32_t* s_vals = (uint32_t*)(s_dyn + 8 * kSortTile);  // tile-sorted values
     uint32_t* s_vin = s_vals + kSortTile;                   // values in load order
@@ -260,10 +261,18 @@ const void* k_sort_pass_ptr() {
     return (const void*)k_sort_pass<ITEMS>;
 }
 
+static int sort_items(int n, int sms) {
+    return n > sms * 8 * kSortThreads ? 16 : n > sms * 2 * kSortThreads ? 8 : kSortMinItems;
+}
+
+size_t sort_zero_words(int n, int sms) {
+    return 8 * 256 + 8 + (size_t)8 * 256 * ceil_div(n > 0 ? n : 1, sort_items(n, sms) * kSortThreads);
+}
+
 // Sort n pairs.  Data starts in (k0, v0); the result ends in (k0, v0) (8
 // passes, even count).  ws: sort_workspace_bytes(capacity) bytes.  When
-// `hist_ready` the 8x256 histograms at the head of ws are already filled (by
-// the fused Morton kernel); otherwise they are computed here.  Returns the
+// `hist_ready` the counting words of ws were zeroed and the 8x256 histograms at
+// their head filled (by the fused Morton kernel); otherwise both is done here.  Returns the
 // first failing status among this call's own memsets and launches (the
 // launches go through cudaLaunchKernelEx, whose return value belongs to that
 // launch alone, so an error left pending by earlier unrelated work is
@@ -274,19 +283,14 @@ cudaError_t sort_pairs(cudaStream_t st, int n, uint64_t* k0, uint32_t* v0, uint6
     uint32_t* hist = (uint32_t*)ws;
     uint32_t* ctr = hist + 8 * 256;
     uint32_t* look = ctr + 8;
-#ifdef NB_SORT_ITEMS
-    const int items = NB_SORT_ITEMS;
-#else
-    const int items = n > sms * 8 * kSortThreads   ? 16
-                      : n > sms * 2 * kSortThreads ? 8
-                                                   : 4;
-#endif
+    const int items = sort_items(n, sms);
     const int tiles = ceil_div(n, items * kSortThreads);
     cudaError_t e;
     cudaLaunchConfig_t cfg = {};
     cfg.stream = st;
     if (!hist_ready) {
-        if ((e = cudaMemsetAsync(hist, 0, sizeof(uint32_t) * 8 * 256, st)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(ws, 0, sizeof(uint32_t) * sort_zero_words(n, sms), st)) != cudaSuccess)
+            return e;
         cfg.gridDim = dim3(min(ceil_div(n, 256 * 8), sms * 8));
         cfg.blockDim = dim3(256);
         cfg.dynamicSmemBytes = 0;
@@ -294,13 +298,15 @@ cudaError_t sort_pairs(cudaStream_t st, int n, uint64_t* k0, uint32_t* v0, uint6
             cudaSuccess)
             return e;
     }
-    if ((e = cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * (8 + (size_t)8 * tiles * 256), st)) !=
-        cudaSuccess)
-        return e;
     uint64_t* ks = k0;
     uint32_t* vs = v0;
     uint64_t* kd = k1;
     uint32_t* vd = v1;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = n <= kEarlyLaunchBodies;
     cfg.gridDim = dim3(tiles);
     cfg.blockDim = dim3(kSortThreads);
     cfg.dynamicSmemBytes = (size_t)items * kSortThreads * 16;

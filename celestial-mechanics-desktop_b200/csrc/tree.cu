@@ -30,14 +30,20 @@
 namespace nb {
 
 constexpr int kMarkThreads = 256;
+// Binary nodes per thread of the marking and numbering kernels: 1, since a
+// node's climb is a chain of dependent loads (20,011 bodies: tree stage 107 ->
+// 85 us against 4), 4 above 2^20 bodies, where the blocks' sums get many.
 constexpr int kMarkItems = 4;
-constexpr int kMarkTile = kMarkThreads * kMarkItems;  // internal nodes per block
+constexpr int kMarkManyNodes = 1 << 20;
+// blocks whose sums a block of the numbering kernel adds up itself; more are
+// scanned by a kernel of their own
+constexpr int kMarkScanBlocks = 4096;
 
 size_t tree_bytes(int cap) {
     size_t c = (size_t)(cap > 1 ? cap : 2);
     size_t b = 0;
     b += 2 * c * 4 + c * 4 + c * 4 + c + c * 4 + c + c * 4 + c * 4;  // binary tree
-    b += (c / kMarkTile + 2) * 4;                                      // block sums
+    b += (c / kMarkThreads + 2) * 4;                                   // block sums
     b += 256;                                                          // align slack
     size_t w = 2 * c;
     b += w * 16 + w * 4 + w * 4 + w * 32 + w * 16 + w * 16 + w * 4 + 16;
@@ -77,7 +83,7 @@ void tree_carve(TreeBufs& t, void* base, int cap) {
     t.bparent = carve<int>(p, c);
     t.child_base = carve<int>(p, c);
     t.walk_index = carve<int>(p, c);
-    t.block_sums = carve<int>(p, c / kMarkTile + 2);
+    t.block_sums = carve<int>(p, c / kMarkThreads + 2);
     t.bdelta = carve<uint8_t>(p, c);
     t.bnchild = carve<uint8_t>(p, c);
     t.capacity = cap;
@@ -93,6 +99,7 @@ __device__ __forceinline__ int prefix_len(const uint64_t* __restrict__ k, int n,
 }
 
 __global__ void k_radix_tree(int n, const uint64_t* __restrict__ keys, TreeBufs t, const int* dn) {
+    pdl_enter();
     n = dev_rows(n, dn);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
@@ -159,13 +166,15 @@ __device__ __forceinline__ bool walk_internal(const TreeBufs& t, int x, int leaf
     return (t.blast[x] - t.bfirst[x] + 1) > leaf_cap && lvl(t, x) < 21;
 }
 
+template <int ITEMS>
 __global__ void __launch_bounds__(kMarkThreads)
 k_octree_mark(int n, TreeBufs t, int leaf_cap, const int* dn) {
     __shared__ int s_red[kMarkThreads / 32];
+    pdl_enter();
     const int m = dev_rows(n, dn) - 1;  // internal nodes (blocks past them sum 0)
     int local = 0;
-    for (int k = 0; k < kMarkItems; k++) {
-        int i = blockIdx.x * kMarkTile + k * kMarkThreads + threadIdx.x;
+    for (int k = 0; k < ITEMS; k++) {
+        int i = (blockIdx.x * ITEMS + k) * kMarkThreads + threadIdx.x;
         if (i >= m) break;
         int P = t.bparent[i];
         int li = lvl(t, i);
@@ -194,11 +203,11 @@ k_octree_mark(int n, TreeBufs t, int leaf_cap, const int* dn) {
     }
 }
 
-// Exclusive scan of the block sums in one block; writes the node count.
-__global__ void k_scan_block_sums(int nblocks, TreeBufs t, int n, const int* dn) {
+// Exclusive scan of the block sums in one block.
+__global__ void k_scan_block_sums(int nblocks, TreeBufs t) {
     __shared__ int s[1024];
-    n = dev_rows(n, dn);
     __shared__ int carry;
+    pdl_enter();
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (int base = 0; base < nblocks; base += 1024) {
@@ -217,17 +226,34 @@ __global__ void k_scan_block_sums(int nblocks, TreeBufs t, int n, const int* dn)
         if (threadIdx.x == 1023) carry += s[1023];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *t.n_nodes = (n >= 2) ? 1 + carry : (n == 1 ? 1 : 0);
 }
 
 // Child slot of every walk-internal node: 1 + exclusive scan of bnchild.
-__global__ void __launch_bounds__(kMarkThreads) k_octree_base(int n, TreeBufs t, const int* dn) {
+// scanned: the block sums are their exclusive scan already; otherwise each
+// block adds up its predecessors'.  The last block writes the node count.
+template <int ITEMS>
+__global__ void __launch_bounds__(kMarkThreads)
+k_octree_base(int n, TreeBufs t, int scanned, const int* dn) {
     __shared__ int s_w[kMarkThreads / 32];
-    const int m = dev_rows(n, dn) - 1;
+    pdl_enter();
+    n = dev_rows(n, dn);
+    const int m = n - 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int off = 1 + t.block_sums[blockIdx.x];
-    for (int k = 0; k < kMarkItems; k++) {
-        int i = blockIdx.x * kMarkTile + k * kMarkThreads + threadIdx.x;
+    int before = 0;
+    if (scanned) {
+        before = t.block_sums[blockIdx.x];
+    } else {
+        for (int b = threadIdx.x; b < (int)blockIdx.x; b += kMarkThreads) before += t.block_sums[b];
+        before = warp_sum(before);
+        if (lane == 0) s_w[warp] = before;
+        __syncthreads();
+        before = 0;
+        for (int w = 0; w < kMarkThreads / 32; w++) before += s_w[w];
+        __syncthreads();
+    }
+    int off = 1 + before;
+    for (int k = 0; k < ITEMS; k++) {
+        int i = (blockIdx.x * ITEMS + k) * kMarkThreads + threadIdx.x;
         int v = (i < m) ? t.bnchild[i] : 0;
         int inc = warp_incl_scan(v);
         if (lane == 31) s_w[warp] = inc;
@@ -242,11 +268,19 @@ __global__ void __launch_bounds__(kMarkThreads) k_octree_base(int n, TreeBufs t,
         off += tot;
         __syncthreads();
     }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+        *t.n_nodes = (n >= 2) ? off : (n == 1 ? 1 : 0);
 }
 
+// Also readies the words that the multipole kernels count in.
 __global__ void k_octree_emit(int n, TreeBufs t, int leaf_cap, const int* dn) {
+    pdl_enter();
     n = dev_rows(n, dn);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        *t.n_leaves = 0;
+        t.counter[0] = 0;
+    }
     if (n == 1) {
         if (i == 0) {
             t.link[0] = make_int4(-1, 0, 0, 1);
@@ -280,6 +314,7 @@ __global__ void k_octree_emit(int n, TreeBufs t, int leaf_cap, const int* dn) {
             t.walk_index[c] = w;
         }
         t.parent_bin[w] = i;
+        t.counter[w] = 0;
         w++;
     });
 }
@@ -344,6 +379,7 @@ __global__ void __launch_bounds__(256)
 k_multipole_leaves(TreeBufs t, const double4* __restrict__ sbody,
                    const float* __restrict__ srad, const double* __restrict__ cube,
                    const uint64_t* __restrict__ skeys, const double* __restrict__ sys_half16) {
+    pdl_enter();
     const int nn = *t.n_nodes;
     for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nn; w += gridDim.x * blockDim.x) {
         const int4 lk = __ldg(&t.link[w]);
@@ -407,6 +443,7 @@ constexpr int kClimbUnroll = NB_CLIMB_UNROLL;
 __global__ void __launch_bounds__(kClimbThreads, NB_CLIMB_MIN_BLOCKS)
 k_multipole_climb(TreeBufs t, const double* __restrict__ cube,
                   const uint64_t* __restrict__ skeys, const double* __restrict__ sys_half16) {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *t.n_leaves) return;
     int p = __ldg(&t.parent_walk[t.leaves[i]]);
@@ -472,21 +509,24 @@ void tree_build(cudaStream_t st, const TreeBufs& t, int n, const uint64_t* skeys
         return;
     }
     const int m = n - 1;
-    const int nblk = ceil_div(m > 0 ? m : 1, kMarkTile);
+    const bool many = n > kMarkManyNodes;
+    const int nblk = ceil_div(m > 0 ? m : 1, kMarkThreads * (many ? kMarkItems : 1));
+    const int scanned = nblk > kMarkScanBlocks;
     if (m > 0) {
-        k_radix_tree<<<ceil_div(m, 256), 256, 0, st>>>(n, skeys, t, dn);
-        k_octree_mark<<<nblk, kMarkThreads, 0, st>>>(n, t, leaf_cap, dn);
+        launch_pdl(n, k_radix_tree, ceil_div(m, 256), 256, 0, st, n, skeys, t, dn);
+        launch_pdl(n, many ? k_octree_mark<kMarkItems> : k_octree_mark<1>, nblk, kMarkThreads, 0, st,
+                   n, t, leaf_cap, dn);
     }
-    k_scan_block_sums<<<1, 1024, 0, st>>>(m > 0 ? nblk : 0, t, n, dn);
-    if (m > 0) k_octree_base<<<nblk, kMarkThreads, 0, st>>>(n, t, dn);
-    k_octree_emit<<<ceil_div(m > 0 ? m : 1, 256), 256, 0, st>>>(n, t, leaf_cap, dn);
-    cudaMemsetAsync(t.counter, 0, sizeof(int) * 2 * (size_t)n, st);
-    cudaMemsetAsync(t.n_leaves, 0, sizeof(int), st);
-    k_multipole_leaves<<<std::min(ceil_div(2 * n, 256), leaves_grid()), 256, 0, st>>>(
-        t, sbody, srad, cube, skeys, sys_half16);
+    if (scanned) launch_pdl(n, k_scan_block_sums, 1, 1024, 0, st, nblk, t);
+    // with m = 0 (one body) there is nothing to number: it writes the node count
+    launch_pdl(n, many ? k_octree_base<kMarkItems> : k_octree_base<1>, m > 0 ? nblk : 1, kMarkThreads,
+               0, st, n, t, scanned, dn);
+    launch_pdl(n, k_octree_emit, ceil_div(m > 0 ? m : 1, 256), 256, 0, st, n, t, leaf_cap, dn);
+    launch_pdl(n, k_multipole_leaves, std::min(ceil_div(2LL * n, 256), leaves_grid()), 256, 0, st, t,
+               sbody, srad, cube, skeys, sys_half16);
     // at most n leaves (each holds a body); the threads past the count return
-    k_multipole_climb<<<ceil_div(n, kClimbThreads), kClimbThreads, 0, st>>>(t, cube, skeys,
-                                                                             sys_half16);
+    launch_pdl(n, k_multipole_climb, ceil_div(n, kClimbThreads), kClimbThreads, 0, st, t, cube, skeys,
+               sys_half16);
 }
 
 }  // namespace nb

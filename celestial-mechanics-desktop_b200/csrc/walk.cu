@@ -312,6 +312,7 @@ template <bool QUAD, bool SHELL, bool POT, bool GUARD, int MAC, int SHAPE = 0, i
 __global__ void __launch_bounds__(WalkShape<MAC, SHAPE, GS>::warps * 32,
                                   WalkShape<MAC, SHAPE, GS>::min_blocks)
 k_walk_group(WalkArgs a) {
+    pdl_enter();
     constexpr int WARPS = WalkShape<MAC, SHAPE, GS>::warps;
     static_assert(!HELP || (MAC == kMacGeometric && !POT), "helping walks");
     __shared__ WalkHelp s_help;
@@ -1154,6 +1155,7 @@ __device__ __forceinline__ double ref_shell(double m, double R, double eps2) {
 template <bool SHELL>
 __global__ void __launch_bounds__(kRefWarps * 32, 4) k_walk_reference(WalkArgs a) {
     __shared__ int2 s_stack[kRefWarps][kRefStack];  // node, body mask
+    pdl_enter();
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int b = lane % kRefBodies, slot = lane / kRefBodies;
@@ -1296,6 +1298,7 @@ __device__ __forceinline__ bool boxes_meet(const Box& a, const Box& b) {
 
 __global__ void k_find_groups(TreeBufs t, int2* __restrict__ groups, int* __restrict__ n_groups,
                               double pack) {
+    pdl_enter();
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= *t.n_nodes) return;
     const int4 lk = t.link[w];
@@ -1351,6 +1354,7 @@ __global__ void k_find_groups(TreeBufs t, int2* __restrict__ groups, int* __rest
 // dense region it does not belong to.
 __global__ void k_find_groups_span(TreeBufs t, int2* __restrict__ groups,
                                    int* __restrict__ n_groups, int span, int size) {
+    pdl_enter();
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= *t.n_nodes) return;
     const int4 lk = t.link[w];
@@ -1362,14 +1366,14 @@ __global__ void k_find_groups_span(TreeBufs t, int2* __restrict__ groups,
 }
 
 void find_groups(cudaStream_t st, const TreeBufs& t, const double4* sbody, int n, int2* groups,
-                 int* n_groups, double pack, int span, int size) {
-    cudaMemsetAsync(n_groups, 0, sizeof(int), st);
+                 int* n_groups, double pack, int span, int size, bool zeroed) {
+    if (!zeroed) cudaMemsetAsync(n_groups, 0, sizeof(int), st);
     if (n <= 0) return;
     if (span >= 32)
-        k_find_groups_span<<<ceil_div(2 * n, 256), 256, 0, st>>>(t, groups, n_groups, span,
-                                                                 size == 64 ? 64 : 32);
+        launch_pdl(n, k_find_groups_span, ceil_div(2LL * n, 256), 256, 0, st, t, groups, n_groups, span,
+                   size == 64 ? 64 : 32);
     else
-        k_find_groups<<<ceil_div(2 * n, 256), 256, 0, st>>>(t, groups, n_groups, pack);
+        launch_pdl(n, k_find_groups, ceil_div(2LL * n, 256), 256, 0, st, t, groups, n_groups, pack);
 }
 
 using WalkKernel = void (*)(WalkArgs);
@@ -1482,46 +1486,44 @@ void walk_group(cudaStream_t st, const WalkConfig& cfg, WalkArgs a, bool quad, b
     // the same bits either way.
     auto help_pays = [&](int warps, int size) { return a.n <= 3LL * warps * size; };
     find_groups(st, a.t, a.sbody, a.n, a.groups, a.n_groups, a.pack, a.group_span,
-                g64 ? 64 : 32);
-    cudaMemsetAsync(a.group_ctr, 0, sizeof(unsigned), st);
+                g64 ? 64 : 32, a.zeroed);
+    if (!a.zeroed) cudaMemsetAsync(a.group_ctr, 0, sizeof(unsigned), st);
+    WalkKernel k;
+    int blocks, warps;
+    size_t smem;
     if (g64) {
-        if (mac == kMacHarvest)
-            k_walk_group<true, false, false, false, kMacHarvest, 0, 64>
-                <<<cfg.blocks64, NB_WALK64_WARPS * 32, kWalkSmem64, st>>>(a);
-        else if (mac == kMacLearned)
-            k_walk_group<true, false, false, false, kMacLearned, 0, 64>
-                <<<cfg.blocks_mac64, kMacWarps64 * 32, kWalkSmemMac64, st>>>(a);
-        else
-            pick_walk64(!(a.eps2 > 0.0), help_pays(cfg.blocks64 * NB_WALK64_WARPS, 64))
-                <<<cfg.blocks64, NB_WALK64_WARPS * 32, kWalkSmem64, st>>>(a);
-        return;
+        blocks = mac == kMacLearned ? cfg.blocks_mac64 : cfg.blocks64;
+        warps = mac == kMacLearned ? kMacWarps64 : NB_WALK64_WARPS;
+        smem = mac == kMacLearned ? kWalkSmemMac64 : kWalkSmem64;
+        if (mac == kMacHarvest) k = k_walk_group<true, false, false, false, kMacHarvest, 0, 64>;
+        else if (mac == kMacLearned) k = k_walk_group<true, false, false, false, kMacLearned, 0, 64>;
+        else k = pick_walk64(!(a.eps2 > 0.0), help_pays(blocks * warps, 64));
+    } else if (mac == kMacLearned) {
+        blocks = cfg.blocks_mac;
+        warps = kMacWarps;
+        smem = kWalkSmemMac;
+        k = k_walk_group<true, false, false, false, kMacLearned>;
+    } else if (mac == kMacGeometric && shape == 1 && quad && !shell && !pot) {
+        blocks = cfg.blocks_small;
+        warps = kWalkWarpsSmall;
+        smem = kWalkWarpsSmall * kWarpFloats * 4;
+        k = a.eps2 > 0.0 ? k_walk_group<true, false, false, false, kMacGeometric, 1>
+                         : k_walk_group<true, false, false, true, kMacGeometric, 1>;
+    } else {
+        blocks = cfg.blocks;
+        warps = kWalkWarps;
+        smem = kWalkSmem;
+        if (mac == kMacHarvest) k = k_walk_group<true, false, false, false, kMacHarvest>;
+        else k = pick_walk(quad, shell, pot, !(a.eps2 > 0.0), help_pays(blocks * warps, 32));
     }
-    if (mac == kMacHarvest) {
-        k_walk_group<true, false, false, false, kMacHarvest>
-            <<<cfg.blocks, kWalkThreads, kWalkSmem, st>>>(a);
-        return;
-    }
-    if (mac == kMacLearned) {
-        k_walk_group<true, false, false, false, kMacLearned>
-            <<<cfg.blocks_mac, kMacWarps * 32, kWalkSmemMac, st>>>(a);
-        return;
-    }
-    if (shape == 1 && quad && !shell && !pot) {
-        const WalkKernel k = a.eps2 > 0.0
-                                 ? k_walk_group<true, false, false, false, kMacGeometric, 1>
-                                 : k_walk_group<true, false, false, true, kMacGeometric, 1>;
-        k<<<cfg.blocks_small, kWalkWarpsSmall * 32, kWalkWarpsSmall * kWarpFloats * 4, st>>>(a);
-        return;
-    }
-    const WalkKernel k = pick_walk(quad, shell, pot, !(a.eps2 > 0.0), help_pays(cfg.blocks * kWalkWarps, 32));
-    k<<<cfg.blocks, kWalkThreads, kWalkSmem, st>>>(a);
+    launch_pdl(a.n, k, blocks, warps * 32, smem, st, a);
 }
 
 void walk_reference(cudaStream_t st, WalkArgs a, bool shell) {
     if (a.n <= 0) return;
     const int blocks = ceil_div(a.n, kRefWarps * kRefBodies);
-    if (shell) k_walk_reference<true><<<blocks, kRefWarps * 32, 0, st>>>(a);
-    else k_walk_reference<false><<<blocks, kRefWarps * 32, 0, st>>>(a);
+    launch_pdl(a.n, shell ? k_walk_reference<true> : k_walk_reference<false>, blocks, kRefWarps * 32, 0,
+               st, a);
 }
 
 }  // namespace nb

@@ -39,7 +39,8 @@ struct WalkArgs {
     unsigned mac_sample;        // groups kept per 65536
     const int* sys_root;        // batched systems: walk-tree root of each system
                                 // (indexed by the key's system field), else null
-    unsigned* group_ctr;        // dynamic group counter (zeroed)
+    unsigned* group_ctr;        // dynamic group counter
+    bool zeroed;                // n_groups and group_ctr are 0 already
     unsigned long long* counters;  // [0] body-cell, [1] body-body interactions
     int* err;
 };
@@ -62,7 +63,7 @@ void walk_init(int sms, WalkConfig& cfg);
 // times the larger part's (0: no packing), plus 32-body slices of level-21
 // buckets that hold more than 32.
 void find_groups(cudaStream_t st, const TreeBufs& t, const double4* sbody, int n, int2* groups,
-                 int* n_groups, double pack, int span, int size = 32);
+                 int* n_groups, double pack, int span, int size = 32, bool zeroed = false);
 size_t walk_front_bytes(const WalkConfig& cfg);
 // Group walk, FP32 monopole(+quadrupole) on FP64-differenced coordinates.
 // mac: 0 geometric, 1 harvest, 2 learned (1 and 2 need quad, no shell, no

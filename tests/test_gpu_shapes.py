@@ -153,3 +153,29 @@ def test_transfers_of_two_threads():
 
     with ThreadPoolExecutor(2) as ex:
         assert all(ex.map(one, (1, 2)))
+
+
+@pytest.mark.parametrize("n", [1, 2, 257, 37888, 37889, 303104, 303105, (1 << 20) + 1])
+def test_keys_and_tree_at_dispatch_edges(engine, oracle, n):
+    """The key kernel's and the node numbering's variants: keys and cube bit
+    for bit, the sorted order stable, and nodes that partition the bodies."""
+    b = scenarios.plummer(n, seed=3)
+    b.active[7::17] = 0
+    keys, _, cube = engine.morton_keys(b.px, b.py, b.pz, b.active, 1)
+    want, _, want_cube = oracle.morton_cube(b.px, b.py, b.pz, b.active)
+    np.testing.assert_array_equal(keys, want)
+    np.testing.assert_array_equal(cube, want_cube)
+    t = engine.build_octree(b.px, b.py, b.pz, b.mass, b.active, 24)
+    order = np.argsort(want, kind="stable")
+    np.testing.assert_array_equal(t["sorted_idx"], order)
+    na = int(b.active.sum())
+    leaf = t["n_children"] == 0
+    assert t["body_count"][0] == na and t["body_count"][leaf].sum() == na
+    first = np.sort(t["body_first"][leaf])
+    np.testing.assert_array_equal(first, np.cumsum(np.r_[0, t["body_count"][leaf][np.argsort(
+        t["body_first"][leaf])]])[:-1])
+    inner = np.flatnonzero(~leaf)
+    m = np.add.reduceat(t["mass"][1:], t["first_child"][inner][np.argsort(
+        t["first_child"][inner])] - 1) if inner.size else np.empty(0)
+    np.testing.assert_allclose(m, t["mass"][inner][np.argsort(t["first_child"][inner])],
+                               rtol=1e-12)
