@@ -655,11 +655,12 @@ NB_API int32_t nb_create(int32_t capacity, int32_t device, nb_engine** out) {
             break;
         if ((r = dalloc(h, &h->scal, 1))) break;
         // a call's arrays up to 256 KB go through the handle's own pinned memory
-        nb::hostio_init(h->io, device, std::min<size_t>(1 << 18, 128 * cap + 8192));
-        if (cudaHostAlloc((void**)&h->scal_host, sizeof(Scal) + 64, cudaHostAllocDefault) != cudaSuccess) {
-            r = fail(h, NB_ERR_CUDA, "pinned scalars");
+        if (!nb::hostio_init(h->io, device)) {
+            r = fail(h, NB_ERR_CUDA, "pinned memory");
             break;
         }
+        static_assert(sizeof(Scal) + sizeof(int) <= nb::kHostExtra, "pinned scalars");
+        h->scal_host = (Scal*)h->io.extra();
         h->nodes_host = (int*)(h->scal_host + 1);
         if (cudaMemset(h->scal, 0, sizeof(Scal)) != cudaSuccess) { r = NB_ERR_CUDA; break; }
         for (auto& e : h->ev)
@@ -679,7 +680,6 @@ NB_API int32_t nb_destroy(nb_engine* h) {
     if (h->st) cudaStreamSynchronize(h->st);
     for (void* p : h->allocs) cudaFree(p);
     nb::hostio_free(h->io);
-    if (h->scal_host) cudaFreeHost(h->scal_host);
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
     if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);

@@ -813,7 +813,10 @@ NB_API int32_t nb_ens_create(int32_t n_systems, const int32_t* sizes, int32_t ds
         nb_ens_destroy(h);
         return r;
     }
-    nb::hostio_init(h->io, device, std::min<size_t>(1 << 18, 80 * n + 8192));
+    if (!nb::hostio_init(h->io, device)) {
+        nb_ens_destroy(h);
+        return NB_ERR_CUDA;
+    }
     *out = h;
     return NB_OK;
 }

@@ -15,11 +15,11 @@
 //     kMaxThreads threads).  A transfer holds the pool for itself; when
 //     another thread's transfer has it, the plain copy is used instead, so
 //     handles never wait for each other.
-// A handle's pinned half is 256 KB at most: 1 MB sends 20,011 bodies 3 %
-// faster and makes their handle 2 ms slower to create.  Before -> now:
-// forces of 2^20 bodies 11.8 -> 8.7 ms a call (5.8 of them on the GPU), of
-// 1,000 bodies 136 -> 90 us, a read-back of 2^20 bodies' state 46 -> 6.3 ms, of
-// an ensemble's 804,337 bodies 25 -> 5.2 ms.
+// Before -> now: forces of 2^20 bodies 11.8 -> 8.7 ms a call (5.8 of them on
+// the GPU), of 1,000 bodies 136 -> 90 us, a read-back of 2^20 bodies' state
+// 46 -> 6.3 ms, of an ensemble's 804,337 bodies 25 -> 5.2 ms.  A closed
+// handle's pinned buffer waits for the next handle (pinning 0.5 MB takes about
+// as long as the rest of a small handle).
 #include "hostio.cuh"
 
 #include <algorithm>
@@ -40,6 +40,10 @@ constexpr size_t kSlotBytes = 1 << 20;
 constexpr size_t kMinChunk = 128 << 10;
 constexpr int kMaxThreads = 7;  // besides the calling one
 constexpr size_t kRowAlign = 256;
+// A handle's pinned half.  1 MB sends 20,011 bodies 3 % faster.
+constexpr size_t kHalfBytes = 256 << 10;
+constexpr size_t kPinBytes = 2 * kHalfBytes + kHostExtra;
+constexpr size_t kMaxSpare = 16;
 
 struct Chunk {
     char* dst;
@@ -53,6 +57,7 @@ struct CopyPool {
     int device = 0;
     int users = 0;
     char* pin = nullptr;
+    std::vector<char*> spare;   // closed handles' pinned buffers (under g_pools_lock)
     cudaEvent_t ev[kSlots] = {};
     bool pending[kSlots] = {};  // an upload's copy out of the slot may still run
     std::mutex busy;            // held for a transfer
@@ -173,6 +178,7 @@ void pool_destroy(CopyPool* p) {
             if (p->pending[k]) cudaEventSynchronize(p->ev[k]);
             cudaEventDestroy(p->ev[k]);
         }
+    for (char* b : p->spare) cudaFreeHost(b);
     if (p->pin) cudaFreeHost(p->pin);
     delete p;
 }
@@ -197,6 +203,7 @@ CopyPool* pool_acquire(int device) {
     }
     const int cpus = (int)std::thread::hardware_concurrency();
     try {
+        p->spare.reserve(kMaxSpare);
         g_pools.push_back(p);
         for (int k = 0; k < std::min(kMaxThreads, cpus / 2 - 1); k++)
             p->threads.emplace_back([p] { p->loop(); });
@@ -254,19 +261,35 @@ size_t packed_bytes(const CopySeg* seg, int n) {
 
 }  // namespace
 
-void hostio_init(HostIO& io, int device, size_t half_bytes) {
-    io.device = device;
-    io.half = padded(half_bytes);
-    if (cudaHostAlloc((void**)&io.pin, 2 * io.half, cudaHostAllocDefault) != cudaSuccess) {
+bool hostio_init(HostIO& io, int device) {
+    try {
+        io.pool = pool_acquire(device);
+    } catch (...) {
+        io.pool = nullptr;
+    }
+    if (io.pool) {
+        std::lock_guard<std::mutex> lk(g_pools_lock);
+        if (!io.pool->spare.empty()) {
+            io.pin = io.pool->spare.back();
+            io.pool->spare.pop_back();
+        }
+    }
+    if (!io.pin && cudaHostAlloc((void**)&io.pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess) {
         io.pin = nullptr;
-        io.half = 0;
         cudaGetLastError();
     }
-    io.pool = pool_acquire(device);
-    if (!io.pool) cudaGetLastError();
+    io.half = kHalfBytes;
+    return io.pin != nullptr;
 }
 
 void hostio_free(HostIO& io) {
+    if (io.pin && io.pool) {
+        std::lock_guard<std::mutex> lk(g_pools_lock);
+        if (io.pool->spare.size() < kMaxSpare) {
+            io.pool->spare.push_back(io.pin);  // capacity was reserved
+            io.pin = nullptr;
+        }
+    }
     if (io.pin) cudaFreeHost(io.pin);
     if (io.pool) pool_release(io.pool);
     io = HostIO();

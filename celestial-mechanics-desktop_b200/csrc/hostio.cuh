@@ -15,17 +15,19 @@ struct CopySeg {
 struct CopyPool;
 
 // A handle's side of the transfers: a pinned buffer of its own for small ones
-// (two halves, up and down, so a call may fill one while the other is read)
-// and its share of the device's copy pool for large ones.
+// (two halves, up and down, so a call may fill one while the other is read,
+// and kHostExtra bytes for the handle's own use) and its share of the device's
+// copy pool for large ones.
+constexpr size_t kHostExtra = 4096;
 struct HostIO {
     char* pin = nullptr;
     size_t half = 0;
-    int device = 0;
     CopyPool* pool = nullptr;
+    char* extra() const { return pin + 2 * half; }
 };
 
-// io is usable (with slower copies) even when this fails.
-void hostio_init(HostIO& io, int device, size_t half_bytes);
+// False: no pinned memory.
+bool hostio_init(HostIO& io, int device);
 void hostio_free(HostIO& io);
 
 // Host arrays to the device in stream order.  On return the host arrays may
