@@ -104,8 +104,11 @@ constexpr int kWalkWarpsSmall = 4;
 #define NB_WALK64_MAC_BLOCKS 4
 #endif
 constexpr int kMacWarps64 = NB_WALK64_MAC_WARPS;
-constexpr int kWalkSmemMac64 = kMacWarps64 * (kWarpFloats + kMacWarpWords) * 4;
-constexpr int kWalkSmem64 = NB_WALK64_WARPS * kWarpFloats * 4;
+// per-warp shared memory of the 64-body walks, in floats: the lists, the
+// lanes' positions (6 x 32) and their compensated sums (12 x 32)
+constexpr int kWarpFloats64 = kCellCap * 10 + kPartCap * 4 + 18 * 32;
+constexpr int kWalkSmemMac64 = kMacWarps64 * (kWarpFloats64 + kMacWarpWords) * 4;
+constexpr int kWalkSmem64 = NB_WALK64_WARPS * kWarpFloats64 * 4;
 static_assert(NB_WALK64_MAC_BLOCKS * (kWalkSmemMac64 + 1024) <= 228 * 1024, "learned walk blocks");
 static_assert(kMacWarps64 <= kWalkWarps && NB_WALK64_WARPS <= kWalkWarps,
               "the stacks are sized for the geometric block shape");
@@ -224,6 +227,7 @@ NB_WALK_EVAL void cells_two(const float* cbuf, int npair, float bx, float by, fl
     const f32x2 BX = pk2(bx, bx), BY = pk2(by, by), BZ = pk2(bz, bz);
     const f32x2 CX = pk2(cx, cx), CY = pk2(cy, cy), CZ = pk2(cz, cz);
     f32x2 TX = 0ull, TY = 0ull, TZ = 0ull, UX = 0ull, UY = 0ull, UZ = 0ull;
+#pragma unroll 2
     for (int m = 0; m < npair; m++) {
         cell_pair_terms<QUAD>(cbuf + m * 20, eps2, BX, BY, BZ, TX, TY, TZ);
         cell_pair_terms<QUAD>(cbuf + m * 20, eps2, CX, CY, CZ, UX, UY, UZ);
@@ -334,27 +338,39 @@ k_walk_group(WalkArgs a) {
     extern __shared__ __align__(16) float s_walk[];
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The 64-body walks keep what only a list flush reads (positions, sums) in
+    // shared memory: 18 registers the traversal has instead (the learned walk no
+    // longer spills; its walk at 2^20 2.47 -> 2.43 ms, ten geometric steps of
+    // 100,003 bodies 9.04 -> 8.68 ms with their transfers).  20 warps per SM at 96
+    // registers, which this would allow, are slower (5.36 -> 5.51 ms at 2^20,
+    // theta 0.5): evaluating a list of cells takes a scheduler 150 cycles per pair
+    // block for two bodies from two warps on (124 of them FMA), so more warps
+    // cannot speed it, and fewer registers slow it.
+    constexpr bool SH = GS == 64;
+    constexpr int kFloats = SH ? kWarpFloats64 : kWarpFloats;
     // Interaction lists in a pair-blocked layout: field f of entry e sits at
     // [(e / 2) * W + 2 f + e % 2], so one 16-byte load returns two fields of
     // entries 2m and 2m+1 as register pairs for the packed f32x2 arithmetic.
     // cells (W = 20): rel x, y, z, -mass, Qxx, Qyy, Qzz, Qxy, Qxz, Qyz
     // bodies (W = 8): rel x, y, z, -mass
-    float* const wbase = s_walk + warp * kWarpFloats;
+    float* const wbase = s_walk + warp * kFloats;
     float* cbuf = wbase;
     float* pbuf = wbase + kCellCap * 10;
     float2* p1 = (float2*)(pbuf + kPartCap * 4);     // R^2, m / (R^2 + eps^2)^1.5
     int* p2 = (int*)(p1 + kPartCap);                 // sorted index (potential walks)
-    int coff = warp * kWarpFloats, poff = coff + kCellCap * 10;  // offsets of cbuf, pbuf (HELP)
+    int coff = warp * kFloats, poff = coff + kCellCap * 10;  // offsets of cbuf, pbuf (HELP)
     // the lanes' bodies, for the helpers: in words that the variant has no
     // other use for (the shell's buffers change hands with their lists)
     constexpr int kPosOff = kCellCap * 10 + kPartCap * (SHELL ? 6 : 4);
-    static_assert(!HELP || (SHELL ? kPartCap : 3 * kPartCap) >= (GS == 64 ? 192 : 96), "positions");
+    static_assert(SH || !HELP || (SHELL ? kPartCap : 3 * kPartCap) >= 96, "positions");
     float* const pos = wbase + kPosOff;
+    __shared__ unsigned long long s_cnt[WARPS][2];  // interactions counted by each warp
+    if (lane < 2) s_cnt[warp][lane] = 0;
     int* fa = a.front + (size_t)(blockIdx.x * WARPS + warp) * a.front_cap;
     const float eps2 = (float)a.eps2;
     const float theta2 = (float)a.theta2;
     const int ngroups = *a.n_groups;
-    unsigned long long cnt_cell = 0, cnt_body = 0, cnt_mlp = 0;
+    unsigned long long cnt_mlp = 0;
     // learned MAC: the network is read through L1 from global memory (11 KB,
     // shared by every block of the SM), rows are staged per warp in shared
     const MacDev* __restrict__ wmac = a.mac;
@@ -362,7 +378,7 @@ k_walk_group(WalkArgs a) {
     float* ys = nullptr;
     int* pend = nullptr;
     if (MAC == kMacLearned) {
-        xs = (uint32_t*)(s_walk + WARPS * kWarpFloats) + warp * kMacWarpWords;
+        xs = (uint32_t*)(s_walk + WARPS * kFloats) + warp * kMacWarpWords;
         ys = (float*)(xs + 32 * 4);
         pend = (int*)(ys + 32);
     }
@@ -452,24 +468,37 @@ k_walk_group(WalkArgs a) {
             }
         }
 
-        float sax = 0.f, say = 0.f, saz = 0.f, cax = 0.f, cay = 0.f, caz = 0.f;
-        float spot = 0.f, cpot = 0.f;
-        // body B's accumulators (groups of more than 32 bodies)
-        float sbx = 0.f, sby = 0.f, sbz = 0.f, cbx = 0.f, cby = 0.f, cbz = 0.f;
-        float spot2 = 0.f, cpot2 = 0.f;
+        // compensated sums: x, y, z of body A (sum, compensation), then of body B
+        float sum_reg[SH ? 1 : 12];
+        float* const sums = SH ? pos + 6 * 32 + lane : sum_reg;
+        constexpr int SS = SH ? 32 : 1;
+#pragma unroll
+        for (int k = 0; k < 12; k++) sums[k * SS] = 0.f;
+        auto add_a = [&](float x, float y, float z) {
+            kahan(sums[0], sums[SS], x);
+            kahan(sums[2 * SS], sums[3 * SS], y);
+            kahan(sums[4 * SS], sums[5 * SS], z);
+        };
+        auto add_b = [&](float x, float y, float z) {
+            kahan(sums[6 * SS], sums[7 * SS], x);
+            kahan(sums[8 * SS], sums[9 * SS], y);
+            kahan(sums[10 * SS], sums[11 * SS], z);
+        };
+        auto total = [&](int k) { return (double)sums[2 * k * SS] - (double)sums[(2 * k + 1) * SS]; };
+        float spot = 0.f, cpot = 0.f, spot2 = 0.f, cpot2 = 0.f;
         int nc = 0, np = 0;
-        unsigned long long grp_entries = 0;  // list entries of this group (load-balance record)
+        unsigned grp_cells = 0, grp_parts = 0;  // list entries of this group
         // lists out with helpers, oldest first: 4 bits each, warp | particles << 3
         unsigned out_fifo = 0;
         int n_out = 0;
         // lists are handed out once so few groups are left that warps may come
         // free before this one ends
         bool can_help = HELP && g + 4 * WARPS * (int)gridDim.x >= ngroups;
-        if (HELP) {
+        if (HELP || SH) {
             pos[lane] = bx;
             pos[32 + lane] = by;
             pos[64 + lane] = bz;
-            if (GS == 64) {
+            if (SH) {
                 pos[96 + lane] = bx2;
                 pos[128 + lane] = by2;
                 pos[160 + lane] = bz2;
@@ -492,14 +521,8 @@ k_walk_group(WalkArgs a) {
             if (ok) {
                 const float* t = s_walk + ((out_fifo & 8) ? ld_shared_volatile(&s_help.parts[w])
                                                           : ld_shared_volatile(&s_help.cells[w]));
-                kahan(sax, cax, t[lane]);
-                kahan(say, cay, t[32 + lane]);
-                kahan(saz, caz, t[64 + lane]);
-                if (GS == 64 && two) {
-                    kahan(sbx, cbx, t[96 + lane]);
-                    kahan(sby, cby, t[128 + lane]);
-                    kahan(sbz, cbz, t[160 + lane]);
-                }
+                add_a(t[lane], t[32 + lane], t[64 + lane]);
+                if (GS == 64 && two) add_b(t[96 + lane], t[128 + lane], t[160 + lane]);
                 __threadfence_block();
                 __syncwarp();
                 if (lane == 0) {
@@ -571,14 +594,6 @@ k_walk_group(WalkArgs a) {
         };
 
         // The cell list's terms on the body at (bx, by, bz) (group-centred).
-        // Both bodies of a two-body lane in one pass over the cell list: each
-        // pair block is read from shared memory once for the two.
-        auto eval_cells2 = [&](float& tx, float& ty, float& tz, float& ux, float& uy, float& uz) {
-            float3 a3, b3;
-            cells_two<QUAD>(cbuf, (nc + 1) >> 1, bx, by, bz, bx2, by2, bz2, eps2, a3, b3);
-            tx = a3.x; ty = a3.y; tz = a3.z;
-            ux = b3.x; uy = b3.y; uz = b3.z;
-        };
         auto eval_cells = [&](float bx, float by, float bz, float& tx, float& ty, float& tz,
                               float& tp) {
             tx = ty = tz = tp = 0.f;
@@ -630,45 +645,38 @@ k_walk_group(WalkArgs a) {
                 }
             }
             if (hand_out(nc, false)) {
-                cnt_cell += (unsigned long long)nc * nvalid;
-                grp_entries += nc;
+                grp_cells += nc;
                 nc = 0;
                 return;
             }
+            // the lanes' bodies
+            const float hx = SH ? pos[lane] : bx, hy = SH ? pos[32 + lane] : by;
+            const float hz = SH ? pos[64 + lane] : bz;
+            const float ix = SH ? pos[96 + lane] : bx2, iy = SH ? pos[128 + lane] : by2;
+            const float iz = SH ? pos[160 + lane] : bz2;
             float tx, ty, tz, tp;
             if (!POT && FUSE2 && two) {
-                float ux, uy, uz;
-                eval_cells2(tx, ty, tz, ux, uy, uz);
+                // one pass over the list: each block is read once for the two
+                float3 t, u;
+                cells_two<QUAD>(cbuf, (nc + 1) >> 1, hx, hy, hz, ix, iy, iz, eps2, t, u);
                 fold_all();
-                kahan(sbx, cbx, ux);
-                kahan(sby, cby, uy);
-                kahan(sbz, cbz, uz);
+                tx = t.x; ty = t.y; tz = t.z;
+                add_b(u.x, u.y, u.z);
             } else {
-                eval_cells(bx, by, bz, tx, ty, tz, tp);
+                eval_cells(hx, hy, hz, tx, ty, tz, tp);
                 fold_all();
                 if (two) {
                     float ux, uy, uz, up;
-                    eval_cells(bx2, by2, bz2, ux, uy, uz, up);
-                    kahan(sbx, cbx, ux);
-                    kahan(sby, cby, uy);
-                    kahan(sbz, cbz, uz);
+                    eval_cells(ix, iy, iz, ux, uy, uz, up);
+                    add_b(ux, uy, uz);
                     if (POT) kahan(spot2, cpot2, up);
                 }
             }
-            kahan(sax, cax, tx);
-            kahan(say, cay, ty);
-            kahan(saz, caz, tz);
+            add_a(tx, ty, tz);
             if (POT) kahan(spot, cpot, tp);
-            cnt_cell += (unsigned long long)nc * nvalid;
-            grp_entries += nc;
+            grp_cells += nc;
             nc = 0;
             __syncwarp();
-        };
-        auto eval_parts2 = [&](float& tx, float& ty, float& tz, float& ux, float& uy, float& uz) {
-            float3 a3, b3;
-            parts_two<GUARD>(pbuf, (np + 1) >> 1, bx, by, bz, bx2, by2, bz2, eps2, a3, b3);
-            tx = a3.x; ty = a3.y; tz = a3.z;
-            ux = b3.x; uy = b3.y; uz = b3.z;
         };
         // The body list's terms on body `self` at (bx, by, bz).
         auto eval_parts = [&](float bx, float by, float bz, int self, float& tx, float& ty,
@@ -712,37 +720,35 @@ k_walk_group(WalkArgs a) {
                 }
             }
             if (hand_out(np, true)) {
-                cnt_body += (unsigned long long)np * nvalid;
-                grp_entries += np;
+                grp_parts += np;
                 np = 0;
                 return;
             }
+            // the lanes' bodies
+            const float hx = SH ? pos[lane] : bx, hy = SH ? pos[32 + lane] : by;
+            const float hz = SH ? pos[64 + lane] : bz;
+            const float ix = SH ? pos[96 + lane] : bx2, iy = SH ? pos[128 + lane] : by2;
+            const float iz = SH ? pos[160 + lane] : bz2;
             float tx, ty, tz, tp;
             if (!SHELL && !POT && FUSE2 && two) {
-                float ux, uy, uz;
-                eval_parts2(tx, ty, tz, ux, uy, uz);
+                float3 t, u;
+                parts_two<GUARD>(pbuf, (np + 1) >> 1, hx, hy, hz, ix, iy, iz, eps2, t, u);
                 fold_all();
-                kahan(sbx, cbx, ux);
-                kahan(sby, cby, uy);
-                kahan(sbz, cbz, uz);
+                tx = t.x; ty = t.y; tz = t.z;
+                add_b(u.x, u.y, u.z);
             } else {
-                eval_parts(bx, by, bz, s, tx, ty, tz, tp);
+                eval_parts(hx, hy, hz, s, tx, ty, tz, tp);
                 fold_all();
                 if (two) {
                     float ux, uy, uz, up;
-                    eval_parts(bx2, by2, bz2, s2, ux, uy, uz, up);
-                    kahan(sbx, cbx, ux);
-                    kahan(sby, cby, uy);
-                    kahan(sbz, cbz, uz);
+                    eval_parts(ix, iy, iz, s2, ux, uy, uz, up);
+                    add_b(ux, uy, uz);
                     if (POT) kahan(spot2, cpot2, up);
                 }
             }
-            kahan(sax, cax, tx);
-            kahan(say, cay, ty);
-            kahan(saz, caz, tz);
+            add_a(tx, ty, tz);
             if (POT) kahan(spot, cpot, tp);
-            cnt_body += (unsigned long long)np * nvalid;
-            grp_entries += np;
+            grp_parts += np;
             np = 0;
             __syncwarp();
         };
@@ -1015,10 +1021,13 @@ k_walk_group(WalkArgs a) {
         if (nc) flush_cells();
         if (np) flush_parts();
         fold_all();
-        if (lane == 0 && a.counters) atomicMax(&a.counters[2], grp_entries);
+        if (lane == 0 && a.counters) {
+            atomicMax(&a.counters[2], (unsigned long long)grp_cells + grp_parts);
+            s_cnt[warp][0] += (unsigned long long)grp_cells * nvalid;
+            s_cnt[warp][1] += (unsigned long long)grp_parts * nvalid;
+        }
         // combine the replicas of each body (lanes equal modulo the width)
-        double fx = (double)sax - (double)cax, fy = (double)say - (double)cay;
-        double fz = (double)saz - (double)caz, fp = (double)spot - (double)cpot;
+        double fx = total(0), fy = total(1), fz = total(2), fp = (double)spot - (double)cpot;
         for (int o = 1 << lw; o < 32; o <<= 1) {
             fx += __shfl_xor_sync(FULL, fx, o);
             fy += __shfl_xor_sync(FULL, fy, o);
@@ -1034,15 +1043,15 @@ k_walk_group(WalkArgs a) {
         }
         if (valid2) {
             const uint32_t row = a.sidx[s2];
-            a.ax[row] = (double)sbx - (double)cbx;
-            a.ay[row] = (double)sby - (double)cby;
-            a.az[row] = (double)sbz - (double)cbz;
+            a.ax[row] = total(3);
+            a.ay[row] = total(4);
+            a.az[row] = total(5);
             if (POT) a.pot[row] = (double)spot2 - (double)cpot2;
         }
     }
     if (lane == 0 && a.counters) {
-        atomicAdd(&a.counters[0], cnt_cell);
-        atomicAdd(&a.counters[1], cnt_body);
+        atomicAdd(&a.counters[0], s_cnt[warp][0]);
+        atomicAdd(&a.counters[1], s_cnt[warp][1]);
         if (MAC == kMacLearned) atomicAdd(&a.counters[3], cnt_mlp);
     }
     if constexpr (HELP) {
@@ -1074,7 +1083,7 @@ k_walk_group(WalkArgs a) {
             }
             __threadfence_block();
             const int shape = ld_shared_volatile(&s_help.shape[warp]);
-            const float* q = s_walk + ld_shared_volatile(&s_help.owner[warp]) * kWarpFloats + kPosOff;
+            const float* q = s_walk + ld_shared_volatile(&s_help.owner[warp]) * kFloats + kPosOff;
             const int entries = shape & 0xFFF, lw = (shape >> 12) & 0xF;
             const int rep = lane >> lw, nrep = 32 >> lw;
             const bool parts = (shape >> 17) & 1;
