@@ -9,47 +9,38 @@
 // replaces the reference GPU gravity_kernel (engine/src/cuda/gravity_kernel.cu:
 // 20-95), which loads inactive sources with their real mass.
 //
-// k_direct_fp32 is the throughput kernel: Morton-sorted targets in tiles of
-// 256 x kD32Per, sources in chunks, one persistent launch over a work queue
-// of (target tile, source chunk) items so the grid ends evenly; j-tiles of
-// 1024 sources arrive raw by cp.async into one of two shared-memory buffers
-// while the previous tile is evaluated, and are converted to FP32
-// coordinates differenced in FP64 against the target tile's centre of mass;
-// kD32Per targets per thread so every broadcast shared-memory read feeds
-// several pair evaluations; a Kahan fold of each j-tile's FP32 partial sum.  The chunk partials are written in FP64
-// and k_direct_reduce adds them in chunk order, so the result does not depend
-// on scheduling.
+// The throughput kernels, k_direct_fp32 and k_direct_fp32_rows: Morton-sorted
+// targets, sources in chunks, one persistent launch over a work queue of
+// (targets, chunk) items so the grid ends evenly; sources arrive raw by
+// cp.async in one of two shared-memory buffers while the previous ones are
+// evaluated, and are converted to FP32 coordinates differenced in FP64 against
+// the centre of mass of the 2560 targets around; several targets per thread so
+// every broadcast shared-memory read feeds several pair evaluations; a Kahan
+// fold of the FP32 partial sum of each j-tile (1024 sources).  The chunk
+// partials are written in FP64 and k_direct_reduce adds them in chunk order, so
+// the result depends neither on scheduling nor on which kernel ran.
+//   * k_direct_fp32: 2560 targets per item, ten per thread, which keeps five
+//     independent packed chains per source in flight and feeds the FMA pipe
+//     best (measured against 4, 6 and 8), one block per SM.
+//   * k_direct_fp32_rows: 256 targets per item, two per thread, five blocks of
+//     128 threads per SM, sources staged 256 at a time: the queue ends evenly
+//     and few bodies spread over all SMs.
 #include <algorithm>
 
 #include "direct.cuh"
 
 namespace nb {
 
-#ifndef NB_D32_THREADS
-#define NB_D32_THREADS 256
-#endif
-constexpr int kD32Threads = NB_D32_THREADS;
-#ifndef NB_D32_PER
-#define NB_D32_PER 10
-#endif
-// targets per thread (even: packed in pairs).  10 keeps five independent
-// packed chains per source in flight at 240 registers (one block of 8 warps
-// per SM); measured against 4 (2 blocks per SM), 6 and 8 it feeds the FMA
-// pipe best.
-constexpr int kD32Per = NB_D32_PER;
-static_assert(kD32Per % 2 == 0, "targets are packed two per f32x2 register");
-// Sources staged per thread per j-tile: 4 (1024-source tiles) measured
-// 70.95 % of FP32 peak against 70.4 % for 1 and 69.9 % for the register
-// prefetch of one source per thread it replaces.
-#ifndef NB_D32_STAGE
-#define NB_D32_STAGE 4
-#endif
-constexpr int kD32Stage = NB_D32_STAGE;              // sources staged per thread per j-tile
-constexpr int kD32Tile = kD32Threads * kD32Stage;    // sources per j-tile
-// dynamic shared memory: two raw FP64 source buffers (cp.async double
-// buffering), their radii, and the converted FP32 tile
-constexpr size_t kD32Smem = 2 * kD32Tile * sizeof(double4) + 2 * kD32Tile * sizeof(float) +
-                            2 * kD32Tile * sizeof(float4) + kD32Tile * sizeof(float2);
+constexpr int kD32Tile = 1024;  // sources per FP32 partial sum (a j-tile)
+constexpr int kD32Threads = 256, kD32Per = 10;
+constexpr int kD32Ref = kD32Threads * kD32Per;      // targets that share a reference point
+constexpr int kD32Stage = kD32Tile / kD32Threads;   // sources staged per thread per j-tile
+constexpr size_t kD32Smem = 2 * kD32Tile * sizeof(double4) + 2 * kD32Tile * sizeof(float4);
+constexpr int kRowThreads = 128, kRowPer = 2, kRowBlocks = 5;
+constexpr int kRowSub = 256;                        // sources staged at a time
+constexpr int kRowTargets = kRowThreads * kRowPer;
+static_assert(kD32Per % 2 == 0 && kRowPer % 2 == 0, "targets are packed two per f32x2 register");
+static_assert(kD32Ref % kRowTargets == 0 && kD32Tile % kRowSub == 0, "rows lie inside one tile");
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -64,11 +55,7 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-constexpr int kD32MinChunk = 4096;    // sources per chunk at least
-#ifndef NB_D32_UNROLL
-#define NB_D32_UNROLL 8
-#endif
-constexpr int kD32Unroll = NB_D32_UNROLL;  // source loop unroll
+constexpr int kD32Unroll = 8;  // source loop unroll
 
 __device__ __forceinline__ void kahan32(float& s, float& c, float x) {
     float y = x - c;
@@ -82,17 +69,14 @@ __device__ __forceinline__ void kahan32(float& s, float& c, float x) {
 // to part[(chunk * 3 + axis) * n + target].  The self pair has
 // dx = dy = dz = 0 and contributes 0 when eps > 0; GUARD (used when
 // eps == 0) zeroes 1/r at r = 0 instead of evaluating 0 * inf.
-template <bool SHELL, bool GUARD>
+template <bool GUARD>
 __global__ void __launch_bounds__(kD32Threads)
-k_direct_fp32(int n, const double4* __restrict__ sbody, const float* __restrict__ srad,
-              float eps2, int n_items, int chunks, int chunk_len, unsigned* __restrict__ ctr,
+k_direct_fp32(int n, const double4* __restrict__ sbody, float eps2, int n_items, int chunks, int chunk_len, unsigned* __restrict__ ctr,
               double* __restrict__ part, unsigned long long* __restrict__ counter) {
     extern __shared__ __align__(16) unsigned char s_d32[];
     double4* raw = (double4*)s_d32;                       // [2][kD32Tile]
-    float* rawR = (float*)(raw + 2 * kD32Tile);           // [2][kD32Tile]
-    float4* sj = (float4*)(rawR + 2 * kD32Tile);
+    float4* sj = (float4*)(raw + 2 * kD32Tile);
     float4* sj2 = sj + kD32Tile;
-    float2* ss = (float2*)(sj2 + kD32Tile);
     __shared__ double s_box[4][kD32Threads / 32];
     __shared__ int s_item;
     for (;;) {
@@ -155,7 +139,6 @@ k_direct_fp32(int n, const double4* __restrict__ sbody, const float* __restrict_
                     double4* dst = raw + buf * kD32Tile + k;
                     cp_async16(dst, &sbody[b0 + k]);
                     cp_async16((char*)dst + 16, (const char*)&sbody[b0 + k] + 16);
-                    if (SHELL) cp_async4(rawR + buf * kD32Tile + k, &srad[b0 + k]);
                 }
             }
             cp_async_commit();
@@ -175,48 +158,21 @@ k_direct_fp32(int n, const double4* __restrict__ sbody, const float* __restrict_
                 const int k = u * kD32Threads + threadIdx.x;
                 const int j = base + k;
                 float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                float R = 0.f;
                 if (j < j1) {
                     const double4 qn = raw[buf * kD32Tile + k];
                     q4 = make_float4((float)(qn.x - ref.x), (float)(qn.y - ref.y),
                                      (float)(qn.z - ref.z), (float)qn.w);
-                    if (SHELL) R = rawR[buf * kD32Tile + k];
                 }
-                if constexpr (SHELL) {
-                    sj[k] = q4;
-                    const float id = rsqrtf(R * R + eps2);
-                    ss[k] = j < j1 ? make_float2(R > 0.f ? R * R : 0.f, q4.w * id * id * id)
-                                   : make_float2(0.f, 0.f);
-                } else {
-                    // each source duplicated into both halves of the packed pairs
-                    sj[k] = make_float4(q4.x, q4.x, q4.y, q4.y);
-                    sj2[k] = make_float4(q4.z, q4.z, q4.w, q4.w);
-                }
+                // each source duplicated into both halves of the packed pairs
+                sj[k] = make_float4(q4.x, q4.x, q4.y, q4.y);
+                sj2[k] = make_float4(q4.z, q4.z, q4.w, q4.w);
             }
             __syncthreads();
             const int cnt = min(kD32Tile, j1 - base);
             float tx[kD32Per], ty[kD32Per], tz[kD32Per];
 #pragma unroll
             for (int u = 0; u < kD32Per; u++) tx[u] = ty[u] = tz[u] = 0.f;
-            if constexpr (SHELL) {
-#pragma unroll 4
-                for (int k = 0; k < cnt; k++) {
-                    const float4 q = sj[k];
-                    const float2 sh = ss[k];
-#pragma unroll
-                    for (int u = 0; u < kD32Per; u++) {
-                        const float dx = bx[u] - q.x, dy = by[u] - q.y, dz = bz[u] - q.z;
-                        const float raw = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        const float r2 = raw + eps2;
-                        const float inv = (GUARD && !(r2 > 0.f)) ? 0.f : rsqrt_ftz(r2);
-                        float f = q.w * (inv * inv * inv);
-                        if (raw < sh.x) f = sh.y;
-                        tx[u] = fmaf(-f, dx, tx[u]);
-                        ty[u] = fmaf(-f, dy, ty[u]);
-                        tz[u] = fmaf(-f, dz, tz[u]);
-                    }
-                }
-            } else {
+            {
                 // two targets per packed instruction; d = q - b, so each half
                 // rounds exactly as fmaf(-f, b - q, t) and fmaf(b - q, b - q, .)
                 constexpr int P = kD32Per / 2;
@@ -278,6 +234,221 @@ k_direct_fp32(int n, const double4* __restrict__ sbody, const float* __restrict_
         if (threadIdx.x == 0 && counter) {
             const int nt = min(kD32Threads * kD32Per, n - t0);
             atomicAdd(counter, (unsigned long long)nt * (unsigned long long)(j1 - j0));
+        }
+    }
+}
+
+// The reference points of the rows: the same sums as above.
+__global__ void __launch_bounds__(kD32Threads)
+k_direct_ref(int n, const double4* __restrict__ sbody, double4* __restrict__ ref) {
+    __shared__ double s_box[4][kD32Threads / 32];
+    const int t0 = blockIdx.x * kD32Ref;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};  // m, m x, m y, m z
+#pragma unroll
+    for (int u = 0; u < kD32Per; u++) {
+        const int i = t0 + u * kD32Threads + threadIdx.x;
+        if (i < n) {
+            const double4 b = sbody[i];
+            acc[0] += b.w;
+            acc[1] += b.w * b.x;
+            acc[2] += b.w * b.y;
+            acc[3] += b.w * b.z;
+        }
+    }
+    for (int k = 0; k < 4; k++)
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xFFFFFFFFu, acc[k], o);
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 4; k++) s_box[k][threadIdx.x >> 5] = acc[k];
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    double m = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
+    for (int w = 0; w < kD32Threads / 32; w++) {
+        m += s_box[0][w];
+        mx += s_box[1][w];
+        my += s_box[2][w];
+        mz += s_box[3][w];
+    }
+    ref[blockIdx.x] = m > 0.0 ? make_double4(mx / m, my / m, mz / m, 0.0) : sbody[t0];
+}
+
+// As k_direct_fp32 over rows of kRowTargets, with the shell theorem too (a
+// source of radius R pulls as a softened shell inside it).
+template <bool SHELL, bool GUARD>
+__global__ void __launch_bounds__(kRowThreads, kRowBlocks)
+k_direct_fp32_rows(int n, const double4* __restrict__ sbody, const float* __restrict__ srad,
+              float eps2, const double4* __restrict__ refs, int n_items, int chunks,
+              int chunk_len, unsigned* __restrict__ ctr, double* __restrict__ part,
+              unsigned long long* __restrict__ counter) {
+    constexpr int PER = kRowPer, kThreads = kRowThreads, kSub = kRowSub;
+    constexpr int kStage = kSub / kThreads;  // sources staged per thread
+    // static shared memory: its constant addresses make the kernel 2 % faster
+    constexpr size_t kBytes = kSub * (2 * sizeof(double4) + 2 * sizeof(float4) +
+                                      (SHELL ? 2 * sizeof(float) + sizeof(float2) : 0));
+    __shared__ __align__(16) unsigned char s_own[kBytes];
+    double4* raw = (double4*)s_own;      // [2][kSub]
+    float4* sj = (float4*)(raw + 2 * kSub);
+    float4* sj2 = sj + kSub;
+    float2* ss = (float2*)(sj2 + kSub);  // shell theorem only, as rawR
+    float* rawR = (float*)(ss + kSub);   // [2][kSub]
+    __shared__ int s_item;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && counter)
+        atomicAdd(counter, (unsigned long long)n * (unsigned long long)n);
+    for (;;) {
+        if (threadIdx.x == 0) s_item = (int)atomicAdd(ctr, 1u);
+        __syncthreads();
+        const int it = s_item;
+        __syncthreads();  // every thread has the item before thread 0 fetches the next
+        if (it >= n_items) break;
+        const int row = it / chunks, chunk = it - row * chunks;
+        const int t0 = row * (kThreads * PER);
+        const int j0 = chunk * chunk_len, j1 = min(n, j0 + chunk_len);
+        const double4 ref = refs[t0 / kD32Ref];
+        float bx[PER], by[PER], bz[PER];
+        float sx[PER], sy[PER], sz[PER], cx[PER], cy[PER], cz[PER];
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int i = t0 + u * kThreads + threadIdx.x;
+            const double4 b = sbody[i < n ? i : n - 1];
+            bx[u] = (float)(b.x - ref.x);
+            by[u] = (float)(b.y - ref.y);
+            bz[u] = (float)(b.z - ref.z);
+            sx[u] = sy[u] = sz[u] = cx[u] = cy[u] = cz[u] = 0.f;
+        }
+        // the next j-tile's raw sources arrive by cp.async while the current
+        // one is evaluated (two raw buffers)
+        auto issue = [&](int b0, int buf) {
+#pragma unroll
+            for (int u = 0; u < kStage; u++) {
+                const int k = u * kThreads + threadIdx.x;
+                if (b0 + k < j1) {
+                    double4* dst = raw + buf * kSub + k;
+                    cp_async16(dst, &sbody[b0 + k]);
+                    cp_async16((char*)dst + 16, (const char*)&sbody[b0 + k] + 16);
+                    if (SHELL) cp_async4(rawR + buf * kSub + k, &srad[b0 + k]);
+                }
+            }
+            cp_async_commit();
+        };
+        issue(j0, 0);
+        int buf = 0;
+        for (int tile = j0; tile < j1; tile += kD32Tile) {
+            float tx[PER], ty[PER], tz[PER];
+            constexpr int P = PER / 2;
+            f32x2 BX[P], BY[P], BZ[P], AX[P], AY[P], AZ[P];
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                BX[p] = pk2(bx[2 * p], bx[2 * p + 1]);
+                BY[p] = pk2(by[2 * p], by[2 * p + 1]);
+                BZ[p] = pk2(bz[2 * p], bz[2 * p + 1]);
+                AX[p] = AY[p] = AZ[p] = 0ull;
+            }
+#pragma unroll
+            for (int u = 0; u < PER; u++) tx[u] = ty[u] = tz[u] = 0.f;
+            const int tile_end = min(tile + kD32Tile, j1);
+            for (int base = tile; base < tile_end; base += kSub, buf ^= 1) {
+                if (base + kSub < j1) {
+                    issue(base + kSub, buf ^ 1);
+                    cp_async_wait<1>();
+                } else {
+                    cp_async_wait<0>();
+                }
+                __syncthreads();  // every thread's copies of these sources have landed
+#pragma unroll
+                for (int u = 0; u < kStage; u++) {
+                    const int k = u * kThreads + threadIdx.x;
+                    const int j = base + k;
+                    float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                    float R = 0.f;
+                    if (j < j1) {
+                        const double4 qn = raw[buf * kSub + k];
+                        q4 = make_float4((float)(qn.x - ref.x), (float)(qn.y - ref.y),
+                                         (float)(qn.z - ref.z), (float)qn.w);
+                        if (SHELL) R = rawR[buf * kSub + k];
+                    }
+                    if constexpr (SHELL) {
+                        sj[k] = q4;
+                        const float id = rsqrtf(R * R + eps2);
+                        ss[k] = j < j1 ? make_float2(R > 0.f ? R * R : 0.f, q4.w * id * id * id)
+                                       : make_float2(0.f, 0.f);
+                    } else {
+                        // each source duplicated into both halves of the packed pairs
+                        sj[k] = make_float4(q4.x, q4.x, q4.y, q4.y);
+                        sj2[k] = make_float4(q4.z, q4.z, q4.w, q4.w);
+                    }
+                }
+                __syncthreads();
+                const int cnt = min(kSub, j1 - base);
+                if constexpr (SHELL) {
+#pragma unroll 4
+                    for (int k = 0; k < cnt; k++) {
+                        const float4 q = sj[k];
+                        const float2 sh = ss[k];
+#pragma unroll
+                        for (int u = 0; u < PER; u++) {
+                            const float dx = bx[u] - q.x, dy = by[u] - q.y, dz = bz[u] - q.z;
+                            const float raw = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                            const float r2 = raw + eps2;
+                            const float inv = (GUARD && !(r2 > 0.f)) ? 0.f : rsqrt_ftz(r2);
+                            float f = q.w * (inv * inv * inv);
+                            if (raw < sh.x) f = sh.y;
+                            tx[u] = fmaf(-f, dx, tx[u]);
+                            ty[u] = fmaf(-f, dy, ty[u]);
+                            tz[u] = fmaf(-f, dz, tz[u]);
+                        }
+                    }
+                } else {
+                    // two targets per packed instruction; d = q - b, so each half
+                    // rounds exactly as fmaf(-f, b - q, t) and fmaf(b - q, b - q, .)
+                    const f32x2 E2 = pk2(eps2, eps2);
+#pragma unroll kD32Unroll
+                    for (int k = 0; k < cnt; k++) {
+                        const float4 qa = sj[k], qb = sj2[k];
+                        const f32x2 qx = pk2(qa.x, qa.y), qy = pk2(qa.z, qa.w);
+                        const f32x2 qz = pk2(qb.x, qb.y), qm = pk2(qb.z, qb.w);
+#pragma unroll
+                        for (int p = 0; p < P; p++) {
+                            const f32x2 dx = sub2(qx, BX[p]), dy = sub2(qy, BY[p]), dz = sub2(qz, BZ[p]);
+                            const f32x2 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, E2)));
+                            float ra, rb;
+                            upk2(r2, ra, rb);
+                            float ia = rsqrt_ftz(ra), ib = rsqrt_ftz(rb);
+                            if (GUARD) {
+                                ia = ra > 0.f ? ia : 0.f;
+                                ib = rb > 0.f ? ib : 0.f;
+                            }
+                            const f32x2 inv = pk2(ia, ib);
+                            const f32x2 f = mul2(mul2(mul2(inv, inv), inv), qm);
+                            AX[p] = fma2(f, dx, AX[p]);
+                            AY[p] = fma2(f, dy, AY[p]);
+                            AZ[p] = fma2(f, dz, AZ[p]);
+                        }
+                    }
+                }
+            }
+            // the j-tile's FP32 sums go into the compensated ones
+            if constexpr (!SHELL) {
+#pragma unroll
+                for (int p = 0; p < P; p++) {
+                    upk2(AX[p], tx[2 * p], tx[2 * p + 1]);
+                    upk2(AY[p], ty[2 * p], ty[2 * p + 1]);
+                    upk2(AZ[p], tz[2 * p], tz[2 * p + 1]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < PER; u++) {
+                kahan32(sx[u], cx[u], tx[u]);
+                kahan32(sy[u], cy[u], ty[u]);
+                kahan32(sz[u], cz[u], tz[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int i = t0 + u * kThreads + threadIdx.x;
+            if (i < n) {
+                part[(size_t)(chunk * 3 + 0) * n + i] = (double)sx[u] - (double)cx[u];
+                part[(size_t)(chunk * 3 + 1) * n + i] = (double)sy[u] - (double)cy[u];
+                part[(size_t)(chunk * 3 + 2) * n + i] = (double)sz[u] - (double)cz[u];
+            }
         }
     }
 }
@@ -600,48 +771,63 @@ cudaError_t direct_fp64_steps(cudaStream_t st, Fp64Args a, bool shell, int order
     return e;
 }
 
+// Bodies up to which k_direct_fp32_rows is the faster one.
+constexpr int kD32RowsMax = 200000;
+
 void direct_fp32(cudaStream_t st, int n, const double4* sbody, const float* srad,
                  const uint32_t* sidx, double eps, bool shell, double* ax, double* ay,
-                 double* az, unsigned long long* counter, void* scratch, size_t scratch_bytes,
+                 double* az, unsigned long long* counter, double* part, double4* ref, int capacity,
                  unsigned* ctr, int sms) {
     if (n <= 0) return;
     const float eps2 = (float)(eps * eps);
-    using K = void (*)(int, const double4*, const float*, float, int, int, int, unsigned*,
-                       double*, unsigned long long*);
-    const K k = eps2 > 0.f ? (shell ? k_direct_fp32<true, false> : k_direct_fp32<false, false>)
-                           : (shell ? k_direct_fp32<true, true> : k_direct_fp32<false, true>);
-    cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kD32Smem);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kD32Threads, kD32Smem);
-    const int resident = sms * (per_sm > 0 ? per_sm : 1);
-    const int tiles = ceil_div(n, kD32Threads * kD32Per);
-    // Chunks per tile: at least 4 waves of items where the scratch and the
-    // kD32MinChunk floor allow, and among those the count whose last wave is
-    // fullest (every item costs the same, so a part-filled last wave idles
-    // the rest of the GPU: 3 chunks of 1024 tiles on 296 resident blocks
-    // leave 62 % of the 11th wave empty, 2 or 4 chunks about 8 %).
-    const long long cmax = std::max<long long>(
-        1, std::min<long long>(std::max(1, ceil_div(n, kD32MinChunk)),
-                               (long long)(scratch_bytes / (sizeof(double) * 3 * (size_t)n))));
-    const long long cmin = std::min<long long>(cmax, std::max(1, ceil_div(4LL * resident, tiles)));
+    // Chunks: from each chunk on the j-tiles start anew, so the chunk length
+    // decides how the FP32 sums round, and it keeps to this rule: items of
+    // kD32Ref targets make at least 4 waves on one block per SM where 4096
+    // sources per chunk and the handle's 290 bytes per body allow it, and among
+    // those counts the fewest chunks within 0.5 % of the fullest last wave.
+    const int tiles = ceil_div(n, kD32Ref);
+    const long long room = 290LL * capacity + (capacity / 1024 + 2) * 4 + 1328;
+    const long long cmax =
+        std::max<long long>(1, std::min<long long>(std::max(1, ceil_div(n, 4096)), room / (24LL * n)));
+    const long long cmin = std::min<long long>(cmax, std::max(1, ceil_div(4LL * sms, tiles)));
     auto fill = [&](long long c) {
         const long long nc = ceil_div(n, ceil_div(n, (int)c));  // chunks actually formed
         const long long it = (long long)tiles * nc;
-        return (double)it / (double)(((it + resident - 1) / resident) * resident);
+        return (double)it / (double)(((it + sms - 1) / sms) * sms);
     };
     double best = 0.0;
     for (long long c = cmin; c <= cmax; c++) best = std::max(best, fill(c));
-    long long chunks = cmin;  // the fewest chunks within 0.5 % of the best fill
+    long long chunks = cmin;
     while (chunks < cmax && fill(chunks) < best - 0.005) chunks++;
     const int chunk_len = ceil_div(n, (int)chunks);
     const int nchunks = ceil_div(n, chunk_len);
-    const int items = tiles * nchunks;
-    cudaMemsetAsync(ctr, 0, sizeof(unsigned), st);
-    k<<<std::min(items, resident), kD32Threads, kD32Smem, st>>>(n, sbody, srad, eps2, items, nchunks,
-                                                         chunk_len, ctr, (double*)scratch,
-                                                         counter);
-    k_direct_reduce<<<ceil_div(n, 256), 256, 0, st>>>(n, nchunks, (const double*)scratch, sidx,
-                                                      ax, ay, az);
+    auto grid = [&](auto kernel, int threads, size_t smem, int items) {
+        if (smem)
+            cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+        return std::min(items, sms * std::max(1, per_sm));
+    };
+    // items of 2560 targets only where they are many waves: k_direct_fp32 against
+    // the rows 301 / 60 us at 2,000 bodies, 590 / 220 at 20,000, 4,820 / 3,980 at
+    // 100,003 (480 items are 3.2 waves and took four), 12.92 / 12.77 ms at
+    // 180,000, 26.3 / 27.0 at 262,144; shells (rows only now) 38.4 / 36.9 there
+    if (!shell && n > kD32RowsMax) {
+        const auto k = eps2 > 0.f ? k_direct_fp32<false> : k_direct_fp32<true>;
+        const int items = tiles * nchunks;
+        k<<<grid(k, kD32Threads, kD32Smem, items), kD32Threads, kD32Smem, st>>>(
+            n, sbody, eps2, items, nchunks, chunk_len, ctr, part, counter);
+    } else {
+        const auto k = eps2 > 0.f
+                           ? (shell ? k_direct_fp32_rows<true, false> : k_direct_fp32_rows<false, false>)
+                           : (shell ? k_direct_fp32_rows<true, true> : k_direct_fp32_rows<false, true>);
+        const int items = ceil_div(n, kRowTargets) * nchunks;
+        k_direct_ref<<<tiles, kD32Threads, 0, st>>>(n, sbody, ref);
+        k<<<grid(k, kRowThreads, 0, items), kRowThreads, 0, st>>>(
+            n, sbody, srad, eps2, ref, items, nchunks, chunk_len, ctr, part, counter);
+    }
+    k_direct_reduce<<<ceil_div(n, 256), 256, 0, st>>>(n, nchunks, part, sidx, ax, ay, az);
 }
 
 }  // namespace nb

@@ -37,11 +37,12 @@ cudaError_t direct_fp64(cudaStream_t st, const Fp64Args& a, bool shell, int orde
 cudaError_t direct_fp64_steps(cudaStream_t st, Fp64Args a, bool shell, int order, int sms,
                               double* const pos[2][3], const double* dts, int n_dt, int steps);
 // FP32 pair math over the n sorted (active) bodies; writes rows sidx[k].
-// scratch: device memory for the per-chunk FP64 partial sums (3 x n doubles
-// per source chunk; at least 24 n bytes); ctr: a device work-queue counter.
+// part: device memory of tree_bytes(capacity) for the chunks' FP64 partial
+// sums; ref: n / 2560 + 1 reference points; ctr: a work-queue counter, 0 before
+// the call.
 void direct_fp32(cudaStream_t st, int n, const double4* sbody, const float* srad,
                  const uint32_t* sidx, double eps, bool shell, double* ax, double* ay,
-                 double* az, unsigned long long* counter, void* scratch, size_t scratch_bytes,
+                 double* az, unsigned long long* counter, double* part, double4* ref, int capacity,
                  unsigned* ctr, int sms);
 
 }  // namespace nb

@@ -7,7 +7,8 @@ import pytest
 
 from conftest import bodies_dict
 from helpers import rel_err
-from nbody_b200 import MODE_BARNES_HUT, MODE_BARNES_HUT_REF, MODE_DIRECT_FP64, scenarios
+from nbody_b200 import (MODE_BARNES_HUT, MODE_BARNES_HUT_REF, MODE_DIRECT, MODE_DIRECT_FP64,
+                        scenarios)
 from nbody_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
@@ -179,3 +180,35 @@ def test_keys_and_tree_at_dispatch_edges(engine, oracle, n):
         t["first_child"][inner])] - 1) if inner.size else np.empty(0)
     np.testing.assert_allclose(m, t["mass"][inner][np.argsort(t["first_child"][inner])],
                                rtol=1e-12)
+
+
+@pytest.mark.parametrize("shell", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 255, 257, 1025, 2561, 4097, 12345])
+def test_fp32_direct_at_row_and_chunk_edges(engine, oracle, n, shell):
+    """Rows of 256 targets, staged 256-source pieces, j-tiles of 1024 and
+    chunks that end inside them: the mode's 2e-6 rms (1e-5 with shells)."""
+    b = scenarios.collisional_disk(n, seed=n, radius_scale=300.0) if shell and n > 1 else \
+        scenarios.plummer(n, seed=n)
+    flags = MODE_DIRECT | (N.FLAG_SHELL_THEOREM if shell else 0)
+    got = engine.compute_forces(b.px, b.py, b.pz, b.mass, b.active, 1e-3, flags, radius=b.radius)
+    want = oracle.direct_forces(b.px, b.py, b.pz, b.mass, b.active, 1e-3, radius=b.radius,
+                                shell=shell)
+    if b.n == 1:
+        assert got[0][0] == got[1][0] == got[2][0] == 0.0
+        return
+    assert np.sqrt(np.mean(rel_err(got, want) ** 2)) < (1e-5 if shell else 2e-6)
+
+
+def test_fp32_direct_on_both_sides_of_the_kernels_rule(engine):
+    """200,000 bodies run the row kernel, one more the tile kernel: each within
+    the mode's 2e-6 rms of the FP64 sum."""
+    b = scenarios.plummer(200_001, seed=5)
+    big = engine.compute_forces(b.px, b.py, b.pz, b.mass, b.active, 1e-3, MODE_DIRECT)
+    exact = engine.compute_forces(b.px, b.py, b.pz, b.mass, b.active, 1e-3, MODE_DIRECT_FP64)
+    small = engine.compute_forces(b.px[:200_000], b.py[:200_000], b.pz[:200_000],
+                                  b.mass[:200_000], b.active[:200_000], 1e-3, MODE_DIRECT)
+    exact_small = engine.compute_forces(b.px[:200_000], b.py[:200_000], b.pz[:200_000],
+                                        b.mass[:200_000], b.active[:200_000], 1e-3,
+                                        MODE_DIRECT_FP64)
+    assert np.sqrt(np.mean(rel_err(big, exact) ** 2)) < 2e-6
+    assert np.sqrt(np.mean(rel_err(small, exact_small) ** 2)) < 2e-6
