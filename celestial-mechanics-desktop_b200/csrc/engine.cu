@@ -235,7 +235,7 @@ int alloc_state(nb_engine* h, nb::State& s, int cap) {
 // scal_host) and the last CUDA error.
 int check_device(nb_engine* h) {
     cudaError_t e = cudaMemcpyAsync(h->scal_host, h->scal, sizeof(Scal), cudaMemcpyDeviceToHost, h->st);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && h->ev_tree)
         e = cudaMemcpyAsync(h->nodes_host, h->tree.n_nodes, sizeof(int), cudaMemcpyDeviceToHost, h->st);
     if (e != cudaSuccess) return fail(h, NB_ERR_CUDA, "error word: %s", cudaGetErrorString(e));
     e = cudaStreamSynchronize(h->st);
