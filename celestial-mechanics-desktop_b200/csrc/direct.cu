@@ -342,8 +342,6 @@ k_direct_fp32_rows(int n, const double4* __restrict__ sbody, const float* __rest
                 BZ[p] = pk2(bz[2 * p], bz[2 * p + 1]);
                 AX[p] = AY[p] = AZ[p] = 0ull;
             }
-#pragma unroll
-            for (int u = 0; u < PER; u++) tx[u] = ty[u] = tz[u] = 0.f;
             const int tile_end = min(tile + kD32Tile, j1);
             for (int base = tile; base < tile_end; base += kSub, buf ^= 1) {
                 if (base + kSub < j1) {
@@ -365,74 +363,63 @@ k_direct_fp32_rows(int n, const double4* __restrict__ sbody, const float* __rest
                                          (float)(qn.z - ref.z), (float)qn.w);
                         if (SHELL) R = rawR[buf * kSub + k];
                     }
-                    if constexpr (SHELL) {
-                        sj[k] = q4;
+                    // each source duplicated into both halves of the packed pairs
+                    sj[k] = make_float4(q4.x, q4.x, q4.y, q4.y);
+                    sj2[k] = make_float4(q4.z, q4.z, q4.w, q4.w);
+                    if (SHELL) {
                         const float id = rsqrtf(R * R + eps2);
                         ss[k] = j < j1 ? make_float2(R > 0.f ? R * R : 0.f, q4.w * id * id * id)
                                        : make_float2(0.f, 0.f);
-                    } else {
-                        // each source duplicated into both halves of the packed pairs
-                        sj[k] = make_float4(q4.x, q4.x, q4.y, q4.y);
-                        sj2[k] = make_float4(q4.z, q4.z, q4.w, q4.w);
                     }
                 }
                 __syncthreads();
                 const int cnt = min(kSub, j1 - base);
-                if constexpr (SHELL) {
-#pragma unroll 4
-                    for (int k = 0; k < cnt; k++) {
-                        const float4 q = sj[k];
-                        const float2 sh = ss[k];
-#pragma unroll
-                        for (int u = 0; u < PER; u++) {
-                            const float dx = bx[u] - q.x, dy = by[u] - q.y, dz = bz[u] - q.z;
-                            const float raw = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                            const float r2 = raw + eps2;
-                            const float inv = (GUARD && !(r2 > 0.f)) ? 0.f : rsqrt_ftz(r2);
-                            float f = q.w * (inv * inv * inv);
-                            if (raw < sh.x) f = sh.y;
-                            tx[u] = fmaf(-f, dx, tx[u]);
-                            ty[u] = fmaf(-f, dy, ty[u]);
-                            tz[u] = fmaf(-f, dz, tz[u]);
-                        }
-                    }
-                } else {
-                    // two targets per packed instruction; d = q - b, so each half
-                    // rounds exactly as fmaf(-f, b - q, t) and fmaf(b - q, b - q, .)
-                    const f32x2 E2 = pk2(eps2, eps2);
+                // two targets per packed instruction; d = q - b, so each half
+                // rounds exactly as fmaf(-f, b - q, t) and fmaf(b - q, b - q, .)
+                const f32x2 E2 = pk2(eps2, eps2);
 #pragma unroll kD32Unroll
-                    for (int k = 0; k < cnt; k++) {
-                        const float4 qa = sj[k], qb = sj2[k];
-                        const f32x2 qx = pk2(qa.x, qa.y), qy = pk2(qa.z, qa.w);
-                        const f32x2 qz = pk2(qb.x, qb.y), qm = pk2(qb.z, qb.w);
+                for (int k = 0; k < cnt; k++) {
+                    const float4 qa = sj[k], qb = sj2[k];
+                    const f32x2 qx = pk2(qa.x, qa.y), qy = pk2(qa.z, qa.w);
+                    const f32x2 qz = pk2(qb.x, qb.y), qm = pk2(qb.z, qb.w);
+                    const float2 sh = SHELL ? ss[k] : make_float2(0.f, 0.f);
 #pragma unroll
-                        for (int p = 0; p < P; p++) {
-                            const f32x2 dx = sub2(qx, BX[p]), dy = sub2(qy, BY[p]), dz = sub2(qz, BZ[p]);
-                            const f32x2 r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, E2)));
-                            float ra, rb;
-                            upk2(r2, ra, rb);
-                            float ia = rsqrt_ftz(ra), ib = rsqrt_ftz(rb);
-                            if (GUARD) {
-                                ia = ra > 0.f ? ia : 0.f;
-                                ib = rb > 0.f ? ib : 0.f;
-                            }
-                            const f32x2 inv = pk2(ia, ib);
-                            const f32x2 f = mul2(mul2(mul2(inv, inv), inv), qm);
-                            AX[p] = fma2(f, dx, AX[p]);
-                            AY[p] = fma2(f, dy, AY[p]);
-                            AZ[p] = fma2(f, dz, AZ[p]);
+                    for (int p = 0; p < P; p++) {
+                        const f32x2 dx = sub2(qx, BX[p]), dy = sub2(qy, BY[p]), dz = sub2(qz, BZ[p]);
+                        f32x2 r2, raw2 = 0ull;
+                        if constexpr (SHELL) {
+                            raw2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                            r2 = add2(raw2, E2);
+                        } else {
+                            r2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, E2)));
                         }
+                        float ra, rb;
+                        upk2(r2, ra, rb);
+                        float ia = rsqrt_ftz(ra), ib = rsqrt_ftz(rb);
+                        if (GUARD) {
+                            ia = ra > 0.f ? ia : 0.f;
+                            ib = rb > 0.f ? ib : 0.f;
+                        }
+                        const f32x2 inv = pk2(ia, ib);
+                        f32x2 f = mul2(mul2(mul2(inv, inv), inv), qm);
+                        if constexpr (SHELL) {
+                            float wa, wb, fa, fb;
+                            upk2(raw2, wa, wb);
+                            upk2(f, fa, fb);
+                            f = pk2(wa < sh.x ? sh.y : fa, wb < sh.x ? sh.y : fb);
+                        }
+                        AX[p] = fma2(f, dx, AX[p]);
+                        AY[p] = fma2(f, dy, AY[p]);
+                        AZ[p] = fma2(f, dz, AZ[p]);
                     }
                 }
             }
             // the j-tile's FP32 sums go into the compensated ones
-            if constexpr (!SHELL) {
 #pragma unroll
-                for (int p = 0; p < P; p++) {
-                    upk2(AX[p], tx[2 * p], tx[2 * p + 1]);
-                    upk2(AY[p], ty[2 * p], ty[2 * p + 1]);
-                    upk2(AZ[p], tz[2 * p], tz[2 * p + 1]);
-                }
+            for (int p = 0; p < P; p++) {
+                upk2(AX[p], tx[2 * p], tx[2 * p + 1]);
+                upk2(AY[p], ty[2 * p], ty[2 * p + 1]);
+                upk2(AZ[p], tz[2 * p], tz[2 * p + 1]);
             }
 #pragma unroll
             for (int u = 0; u < PER; u++) {
@@ -812,7 +799,7 @@ void direct_fp32(cudaStream_t st, int n, const double4* sbody, const float* srad
     // items of 2560 targets only where they are many waves: k_direct_fp32 against
     // the rows 301 / 60 us at 2,000 bodies, 590 / 220 at 20,000, 4,820 / 3,980 at
     // 100,003 (480 items are 3.2 waves and took four), 12.92 / 12.77 ms at
-    // 180,000, 26.3 / 27.0 at 262,144; shells (rows only now) 38.4 / 36.9 there
+    // 180,000, 26.3 / 27.0 at 262,144; shells (rows only now) 38.4 / 34.6 there
     if (!shell && n > kD32RowsMax) {
         const auto k = eps2 > 0.f ? k_direct_fp32<false> : k_direct_fp32<true>;
         const int items = tiles * nchunks;
