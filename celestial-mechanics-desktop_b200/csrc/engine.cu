@@ -176,6 +176,7 @@ struct nb_engine {
     } cmerge{};
     bool ev_valid = false;
     bool ev_tree = false;
+    bool no_counts = false;    // the last evaluation counts nothing on the device
     bool ev_collide = false;   // ev[4], ev[5] bracket the last collision stage
     bool tree_current = false; // the last force evaluation left a tree (with radii) of the
                                // current positions: keys0/vals0, sbody/srad, tree, cube
@@ -382,8 +383,7 @@ int force_pipeline(nb_engine* h, int flags, double eps, bool kick, double dt,
     if (mode != NB_MODE_DIRECT_FP64 || kick)
         nb::launch_kick_drift_bbox(h->st, n, h->s, kick, dt, box_bufs(h), force_words(h, n),
                                    sc->err, dn);
-    if (mode == NB_MODE_DIRECT_FP64)
-        cudaMemsetAsync(sc->counters, 0, sizeof(sc->counters), h->st);
+    h->no_counts = mode == NB_MODE_DIRECT_FP64;
     const int* dna = dn ? &sc->n_active : nullptr;
     if (dn && mode != NB_MODE_BARNES_HUT)
         return fail(h, NB_ERR_INVALID_ARG, "device row counts need NB_MODE_BARNES_HUT");
@@ -540,7 +540,8 @@ int step_graph(nb_engine* h, int flags, double dt, double eps) {
 
 // Counters of the last evaluation, from the scalars of the last check.
 void collect_counters(nb_engine* h) {
-    const unsigned long long* c = h->scal_host->counters;
+    static const unsigned long long none[4] = {0, 0, 0, 0};
+    const unsigned long long* c = h->no_counts ? none : h->scal_host->counters;
     h->counters[NB_C_CELL_INTERACTIONS] = (int64_t)c[0];
     h->counters[NB_C_BODY_INTERACTIONS] = (int64_t)c[1];
     h->counters[NB_C_MAX_GROUP_WORK] = (int64_t)c[2];
@@ -565,10 +566,11 @@ int count_active_host(const uint8_t* a, int n) {
 
 // Upload positions / masses / radii / active into the device rows (the
 // host-array entry points stage through the state arrays).  `more` arrays
-// travel with them.  A null mass or radius array leaves zeros.
+// travel with them.  A null mass or radius array leaves zeros (no_radii: the
+// radii are not read, and stay what they were).
 int stage_bodies(nb_engine* h, int n, const double* px, const double* py, const double* pz,
                  const double* mass, const double* radius, const uint8_t* active,
-                 const Segs* more = nullptr) {
+                 const Segs* more = nullptr, bool no_radii = false) {
     int r;
     if ((r = check_n(h, n))) return r;
     if (n > 0 && (!px || !py || !pz || !active))
@@ -585,7 +587,7 @@ int stage_bodies(nb_engine* h, int n, const double* px, const double* py, const 
     s.add(h->s.active, active, (size_t)n);
     if ((r = send(h, s))) return r;
     if (!mass) NB_CUDA(h, cudaMemsetAsync(h->s.mass, 0, d, h->st));
-    if (!radius) NB_CUDA(h, cudaMemsetAsync(h->s.radius, 0, d, h->st));
+    if (!radius && !no_radii) NB_CUDA(h, cudaMemsetAsync(h->s.radius, 0, d, h->st));
     h->n = n;
     h->n_active = n > 0 ? count_active_host(active, n) : 0;
     h->has_state = false;
@@ -834,9 +836,10 @@ NB_API int32_t nb_compute_forces(nb_engine* h, int32_t n, const double* px, cons
     if (!mass && n > 0) return fail(h, NB_ERR_INVALID_ARG, "null mass array");
     if (n > 0 && (!ax || !ay || !az)) return fail(h, NB_ERR_INVALID_ARG, "null output array");
     int r;
-    // only the shell theorem reads radii here
-    if ((r = stage_bodies(h, n, px, py, pz, mass,
-                          (flags & NB_FLAG_SHELL_THEOREM) ? radius : nullptr, active)))
+    // only the shell theorem reads radii here; a tree for collisions carries zeros
+    const bool shell = (flags & NB_FLAG_SHELL_THEOREM) != 0;
+    if ((r = stage_bodies(h, n, px, py, pz, mass, shell ? radius : nullptr, active, nullptr,
+                          !shell && !(flags & NB_FLAG_COLLISIONS))))
         return r;
     if (n == 0) return NB_OK;
     if ((r = force_pipeline(h, flags, softening, false, 0.0))) return r;
@@ -1034,6 +1037,7 @@ int run_collide_graphs(nb_engine* h, int n_steps, double dt, double eps, int fla
     }
     NB_CUDA(h, cudaMemcpyAsync(&h->scal->n_rows, &h->n, sizeof(int), cudaMemcpyHostToDevice,
                                h->st));
+    h->no_counts = false;
     const int first = h->s.px == h->cstate[0] ? 0 : 1;
     for (int k = 0; k < n_steps; k++)
         NB_CUDA(h, cudaGraphLaunch(h->cgraph[(first + k) & 1], h->st));
@@ -1068,7 +1072,7 @@ int run_steps(nb_engine* h, int n_steps, double dt, double softening, int flags)
                                    {h->s_alt.px, h->s_alt.py, h->s_alt.pz}};
         h->tree_current = false;
         h->ev_tree = false;
-        NB_CUDA(h, cudaMemsetAsync(h->scal->counters, 0, sizeof(h->scal->counters), h->st));
+        h->no_counts = true;
         for (int k = 0; k < 3; k++) record(h, k);
         NB_CUDA(h, nb::direct_fp64_steps(h->st, fp64_args(h, softening),
                                          (flags & NB_FLAG_SHELL_THEOREM) != 0, fp64_order(flags),
@@ -1083,6 +1087,7 @@ int run_steps(nb_engine* h, int n_steps, double dt, double softening, int flags)
         // Multi-step calls replay one captured step (a CUDA graph) n times;
         // the row and active counts do not change without collisions.
         if ((r = step_graph(h, flags, dt, softening))) return r;
+        h->no_counts = false;
         for (int k = 0; k < n_steps; k++)
             NB_CUDA(h, cudaGraphLaunch(h->graph_exec, h->st));
         if ((r = check_device(h))) return r;

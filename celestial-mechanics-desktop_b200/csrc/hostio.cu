@@ -10,15 +10,15 @@
 //     per call.
 //   * A large one is cut into chunks that a pool of threads moves through a
 //     ring of pinned slots, so the host copies run side by side and overlap
-//     the bus.  There is one pool per device, made with the device's first
-//     handle and given back with its last (kSlots MB pinned, at most
-//     kMaxThreads threads).  A transfer holds the pool for itself; when
-//     another thread's transfer has it, the plain copy is used instead, so
-//     handles never wait for each other.
-// Before -> now: forces of 2^20 bodies 11.8 -> 8.7 ms a call (5.8 of them on
-// the GPU), of 1,000 bodies 136 -> 90 us, a read-back of 2^20 bodies' state
+//     the bus.  There is one pool per device; its slots (kSlots MB pinned) and
+//     threads (at most kMaxThreads) come when kPoolAfter bytes have gone the
+//     plain way, and go with the device's last handle.  A transfer holds the
+//     pool for itself; when another thread's transfer has it, the plain copy
+//     is used instead, so handles never wait for each other.
+// Before -> now: forces of 2^20 bodies 11.8 -> 8.4 ms a call (5.4 of them on
+// the GPU), of 1,000 bodies 136 -> 82 us, a read-back of 2^20 bodies' state
 // 46 -> 6.3 ms, of an ensemble's 804,337 bodies 25 -> 5.2 ms.  A closed
-// handle's pinned buffer waits for the next handle (pinning 0.5 MB takes about
+// handle's pinned buffer waits for the next handle (pinning 1 MB takes 1 to 4 ms,
 // as long as the rest of a small handle).
 #include "hostio.cuh"
 
@@ -40,10 +40,18 @@ constexpr size_t kSlotBytes = 1 << 20;
 constexpr size_t kMinChunk = 128 << 10;
 constexpr int kMaxThreads = 7;  // besides the calling one
 constexpr size_t kRowAlign = 256;
-// A handle's pinned half.  1 MB sends 20,011 bodies 3 % faster.
-constexpr size_t kHalfBytes = 256 << 10;
+// A handle's pinned half.  The forces of 20,011 bodies (0.66 MB up, 0.48 MB
+// down) take 0.48 ms a call, with 256 KB 0.52 and with 1 MB 0.50.
+constexpr size_t kHalfBytes = 512 << 10;
+// The pool takes transfers from these sizes on, where its threads' wake-up is
+// paid for: 7.6 MB up before ten steps of 100,000 bodies 8.7 ms in all against
+// 9.2 plain, 4.8 MB down 0.42 against 0.82.
+constexpr size_t kPoolUp = 4 << 20, kPoolDown = 2 << 20;
+// Pinning the slots takes 14 ms, what the plain copy of this much costs more
+// than the pool's: a program that moves less never pays for them.
+constexpr size_t kPoolAfter = 32 << 20;
 constexpr size_t kPinBytes = 2 * kHalfBytes + kHostExtra;
-constexpr size_t kMaxSpare = 16;
+constexpr size_t kMaxSpare = 8;
 
 struct Chunk {
     char* dst;
@@ -76,6 +84,8 @@ struct CopyPool {
     bool open = false;  // the job still takes threads
     int inside = 0;     // threads at work on it
     bool stop = false;
+    bool made = false;  // slots, events and threads (under busy)
+    size_t moved = 0;   // bytes that went the plain way before that (under busy)
 
     // Chunk c goes through slot c % kSlots when the slot's earlier chunks have
     // left it (up: its copy was enqueued, and its event says when it ended;
@@ -127,8 +137,33 @@ struct CopyPool {
         }
     }
 
-    // A pool of one or two threads moves no more than the plain copy does.
-    bool useful() const { return threads.size() >= 2; }
+    // Slots, events and threads, once kPoolAfter bytes have gone without (busy
+    // held).  A pool of one or two threads moves no more than the plain copy
+    // does: false then, and where there is no pinned memory to be had.
+    bool ready(size_t total) {
+        if (!made) {
+            moved += total;
+            if (moved < kPoolAfter) return false;
+            made = true;
+            // another thread of the program may be capturing a graph
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            bool ok = cudaHostAlloc((void**)&pin, kSlots * kSlotBytes, cudaHostAllocDefault) ==
+                      cudaSuccess;
+            for (int k = 0; ok && k < kSlots; k++)
+                ok = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming) == cudaSuccess;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            const int cpus = (int)std::thread::hardware_concurrency();
+            try {
+                for (int k = 0; ok && k < std::min(kMaxThreads, cpus / 2 - 1); k++)
+                    threads.emplace_back([this] { loop(); });
+            } catch (...) {
+                // fewer threads, or none: the calling thread does the rest
+            }
+            if (!ok) cudaGetLastError();
+        }
+        return threads.size() >= 2;
+    }
 
     // The whole transfer, with `busy` held.  Returns when every host array has
     // been read or written.
@@ -194,25 +229,12 @@ CopyPool* pool_acquire(int device) {
     if (!p) return nullptr;
     p->device = device;
     p->users = 1;
-    bool ok = cudaHostAlloc((void**)&p->pin, kSlots * kSlotBytes, cudaHostAllocDefault) == cudaSuccess;
-    for (int k = 0; ok && k < kSlots; k++)
-        ok = cudaEventCreateWithFlags(&p->ev[k], cudaEventDisableTiming) == cudaSuccess;
-    if (!ok) {
-        pool_destroy(p);
-        return nullptr;
-    }
-    const int cpus = (int)std::thread::hardware_concurrency();
     try {
         p->spare.reserve(kMaxSpare);
         g_pools.push_back(p);
-        for (int k = 0; k < std::min(kMaxThreads, cpus / 2 - 1); k++)
-            p->threads.emplace_back([p] { p->loop(); });
     } catch (...) {
-        // fewer threads, or none: the calling thread does the rest
-        if (g_pools.empty() || g_pools.back() != p) {
-            pool_destroy(p);
-            return nullptr;
-        }
+        pool_destroy(p);
+        return nullptr;
     }
     return p;
 }
@@ -299,11 +321,12 @@ namespace {
 
 // Through the pool, if it is there and free; nothing is thrown on.
 bool by_pool(HostIO& io, bool up, cudaStream_t st, const CopySeg* seg, int n, cudaError_t* e) {
-    if (!io.pool || !io.pool->useful()) return false;
+    const size_t total = total_bytes(seg, n);
+    if (!io.pool || total < (up ? kPoolUp : kPoolDown)) return false;
     try {
         std::unique_lock<std::mutex> lk(io.pool->busy, std::try_to_lock);
-        if (!lk.owns_lock()) return false;
-        *e = io.pool->run(up, st, seg, n, total_bytes(seg, n));
+        if (!lk.owns_lock() || !io.pool->ready(total)) return false;
+        *e = io.pool->run(up, st, seg, n, total);
         return true;
     } catch (...) {
         return false;
