@@ -319,14 +319,38 @@ void hostio_free(HostIO& io) {
 
 namespace {
 
-// Through the pool, if it is there and free; nothing is thrown on.
+// An array the caller pinned moves at the bus rate by itself; through the
+// slots 2^20 bodies' forces from pinned arrays took 5.3 ms instead of 3.8.
+bool pageable(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// The pageable arrays of a large transfer through the pool, if it is there and
+// free, the others by plain copies; false: nothing was done.  Nothing is
+// thrown on.
 bool by_pool(HostIO& io, bool up, cudaStream_t st, const CopySeg* seg, int n, cudaError_t* e) {
-    const size_t total = total_bytes(seg, n);
-    if (!io.pool || total < (up ? kPoolUp : kPoolDown)) return false;
+    const size_t least = up ? kPoolUp : kPoolDown;
+    if (!io.pool || total_bytes(seg, n) < least) return false;
     try {
+        std::vector<CopySeg> own, rest;
+        for (int i = 0; i < n; i++)
+            (pageable(up ? seg[i].src : seg[i].dst) ? rest : own).push_back(seg[i]);
+        const size_t total = total_bytes(rest.data(), (int)rest.size());
+        if (total < least) return false;
         std::unique_lock<std::mutex> lk(io.pool->busy, std::try_to_lock);
         if (!lk.owns_lock() || !io.pool->ready(total)) return false;
-        *e = io.pool->run(up, st, seg, n, total);
+        for (const CopySeg& k : own) {
+            *e = cudaMemcpyAsync(k.dst, k.src, k.bytes,
+                                 up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st);
+            if (*e != cudaSuccess) return true;
+        }
+        *e = io.pool->run(up, st, rest.data(), (int)rest.size(), total);
+        if (!up && !own.empty() && *e == cudaSuccess) *e = cudaStreamSynchronize(st);
         return true;
     } catch (...) {
         return false;

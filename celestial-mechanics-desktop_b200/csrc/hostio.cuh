@@ -30,8 +30,8 @@ struct HostIO {
 bool hostio_init(HostIO& io, int device);
 void hostio_free(HostIO& io);
 
-// Host arrays to the device in stream order.  On return the host arrays may
-// be changed.  An earlier upload through the same handle has to have ended.
+// Host arrays to the device in stream order.  Pageable arrays may be changed on
+// return, pinned ones when the stream has been synchronised.  An earlier upload through the same handle has to have ended.
 cudaError_t copy_up(HostIO& io, cudaStream_t st, const CopySeg* seg, int n);
 
 // Device arrays to the host.  start_down enqueues what fits the pinned half

@@ -136,6 +136,28 @@ def test_state_round_trip_at_transfer_sizes(engine, n):
     np.testing.assert_array_equal(ids, np.arange(n))
 
 
+@pytest.mark.parametrize("n", [30000, 120001, 300001])
+@pytest.mark.parametrize("fields", ["px py pz mass", "px py pz vx vy vz mass radius ax ay az", "vz"])
+def test_state_round_trip_from_pinned_arrays(engine, n, fields):
+    """Pinned arrays among pageable ones, at sizes that go by the pool: every
+    array comes back bit for bit."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    b = scenarios.plummer(n, seed=n)
+    for k in ("ax", "ay", "az"):
+        setattr(b, k, rng.standard_normal(n))
+    keep = {k: torch.from_numpy(np.ascontiguousarray(getattr(b, k))).pin_memory()
+            for k in fields.split()}
+    for k, t in keep.items():
+        setattr(b, k, t.numpy())
+    for _ in range(3):
+        engine.set_state(b)
+        s, _ = engine.get_state()
+        for k in ("px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az", "mass", "radius"):
+            np.testing.assert_array_equal(getattr(s, k), getattr(b, k), err_msg=k)
+
+
 def test_transfers_of_two_threads():
     """Two handles in two threads share the copy pool: each gets its own data."""
     from concurrent.futures import ThreadPoolExecutor
