@@ -720,9 +720,9 @@ def run_theta05(args, ws, rank, local):
                              "frac": achieved / fp32_peak, "flop_per_pair": FLOPS_BODY,
                              "traffic": (walk_traffic_per_launch()
                                          if n == N_BODIES and not direct else None)},
-                # direct: kick-drift, cube, keys, 8 passes, gather, zero-acc,
-                # the direct sum, its chunk reduction, kick
-                "gpu_launches": (16 if direct else launches_per_step()) * args.steps,
+                # direct: kick-drift, keys, 8 passes, gather, the direct sum,
+                # its chunk reduction, kick
+                "gpu_launches": (14 if direct else launches_per_step()) * args.steps,
                 "clocks": arm["clocks"]}
         if direct and ws == 1 and not args.no_cpu_baseline:
             # the CpuParallelBackend restatement (FP64, OpenMP over targets) on
@@ -746,8 +746,8 @@ def run_theta05(args, ws, rank, local):
 
 ENS_SYSTEMS, ENS_SEED, ENS_DS_MAX, ENS_DT = 512, 3, 2048, 1e-4
 # kernels of one ensemble step: kick-drift, direct work queue, cubes, keys,
-# 8 sort passes, gather, tree (radix, mark, scan, base, emit, multipoles),
-# system roots (2), walk groups, walk, kick
+# 8 sort passes, gather, tree (radix, mark, base, emit, multipole leaves and
+# climb), system roots (2), walk groups, walk, kick
 ENS_LAUNCHES_PER_STEP = 1 + 1 + 1 + 1 + 8 + 1 + 6 + 2 + 1 + 1 + 1
 
 
@@ -965,11 +965,11 @@ def run_compact(args, ws, rank, local):
 
 
 def launches_per_step() -> int:
-    """Kernels of one geometric device step: kick-drift-bbox, cube, keys, 8
-    sort passes, gather, zero-acc, radix tree, octree mark, block scan,
-    octree base, octree emit, multipole leaves, multipole climb, walk
-    groups, walk, kick (the learned MAC adds its per-node screen terms)."""
-    return 1 + 1 + 1 + 8 + 1 + 1 + 5 + 2 + 1 + 1 + 1
+    """Kernels of one geometric device step: kick-drift-bbox, keys, 8 sort
+    passes, gather, radix tree, octree mark, octree base, octree emit,
+    multipole leaves, multipole climb, walk groups, walk, kick (the learned
+    MAC adds its per-node screen terms)."""
+    return 1 + 1 + 8 + 1 + 4 + 2 + 1 + 1 + 1
 
 
 def _timed_steps(eng, stream, steps, dt, eps, flags, dev, ws):
@@ -1047,7 +1047,8 @@ def run_ds1000(args, ws, rank, local):
                     "value": steps / cpu_s, "unit": "steps/s", "cores": threads, "kind": "port",
                     "sample": f"the same {steps} steps with the CpuParallelBackend restatement "
                               "(OpenMP over targets)"},
-                "clocks": clk, "gpu_launches": 5 * steps}
+                # one kernel per step, and the opening kick and drift
+                "clocks": clk, "gpu_launches": steps + 1}
     eng.close()
     return line
 
