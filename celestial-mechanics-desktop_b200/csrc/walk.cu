@@ -105,9 +105,11 @@ constexpr int kWalkWarpsSmall = 4;
 #endif
 constexpr int kMacWarps64 = NB_WALK64_MAC_WARPS;
 // per-warp shared memory of the 64-body walks, in floats: the lists, the
-// lanes' positions (6 x 32) and their compensated sums (12 x 32)
-constexpr int kWarpFloats64 = kCellCap * 10 + kPartCap * 4 + 18 * 32;
-constexpr int kWalkSmemMac64 = kMacWarps64 * (kWarpFloats64 + kMacWarpWords) * 4;
+// lanes' positions (6 x 32) and, in the geometric ones, their compensated sums
+// (12 x 32)
+constexpr int kWarpFloatsMac64 = kCellCap * 10 + kPartCap * 4 + 6 * 32;
+constexpr int kWarpFloats64 = kWarpFloatsMac64 + 12 * 32;
+constexpr int kWalkSmemMac64 = kMacWarps64 * (kWarpFloatsMac64 + kMacWarpWords) * 4;
 constexpr int kWalkSmem64 = NB_WALK64_WARPS * kWarpFloats64 * 4;
 static_assert(NB_WALK64_MAC_BLOCKS * (kWalkSmemMac64 + 1024) <= 228 * 1024, "learned walk blocks");
 static_assert(kMacWarps64 <= kWalkWarps && NB_WALK64_WARPS <= kWalkWarps,
@@ -371,15 +373,19 @@ k_walk_group(WalkArgs a) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // The 64-body walks keep what only a list flush reads (positions, sums) in
-    // shared memory: 18 registers the traversal has instead (the learned walk no
-    // longer spills; its walk at 2^20 2.47 -> 2.43 ms, ten geometric steps of
-    // 100,003 bodies 9.04 -> 8.68 ms with their transfers).  20 warps per SM at 96
+    // shared memory: 18 registers the traversal has instead (ten geometric steps
+    // of 100,003 bodies 9.04 -> 8.68 ms with their transfers).  The learned walk
+    // keeps its sums in registers: without the six of the positions it no longer
+    // spills, and reading the sums back costs more than they free (at 2^20 and
+    // rms 9.8e-4, ms: all in registers 2.06, positions out 2.04, sums out 2.06,
+    // both 2.14 against 2.08 before).  20 warps per SM at 96
     // registers, which this would allow, are slower (5.36 -> 5.51 ms at 2^20,
     // theta 0.5): evaluating a list of cells takes a scheduler 150 cycles per pair
     // block for two bodies from two warps on (124 of them FMA), so more warps
     // cannot speed it, and fewer registers slow it.
-    constexpr bool SH = GS == 64;
-    constexpr int kFloats = SH ? kWarpFloats64 : kWarpFloats;
+    constexpr bool SH = GS == 64;                          // positions
+    constexpr bool SUMS = SH && MAC != kMacLearned;        // sums
+    constexpr int kFloats = SUMS ? kWarpFloats64 : SH ? kWarpFloatsMac64 : kWarpFloats;
     // Interaction lists in a pair-blocked layout: field f of entry e sits at
     // [(e / 2) * W + 2 f + e % 2], so one 16-byte load returns two fields of
     // entries 2m and 2m+1 as register pairs for the packed f32x2 arithmetic.
@@ -501,9 +507,9 @@ k_walk_group(WalkArgs a) {
         }
 
         // compensated sums: x, y, z of body A (sum, compensation), then of body B
-        float sum_reg[SH ? 1 : 12];
-        float* const sums = SH ? pos + 6 * 32 + lane : sum_reg;
-        constexpr int SS = SH ? 32 : 1;
+        float sum_reg[SUMS ? 1 : 12];
+        float* const sums = SUMS ? pos + 6 * 32 + lane : sum_reg;
+        constexpr int SS = SUMS ? 32 : 1;
 #pragma unroll
         for (int k = 0; k < 12; k++) sums[k * SS] = 0.f;
         auto add_a = [&](float x, float y, float z) {
