@@ -363,27 +363,35 @@ __global__ void k_ens_energy(int n, const int* __restrict__ sys_of_all, const in
     }
 }
 
+// A non-finite word among the `words` sets the error word.
+__global__ void k_check_finite(size_t words, const double* __restrict__ v, int* err) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += stride)
+        if (!isfinite(v[i])) dev_flag(err, kErrNonFinite);
+}
+
 // Up to nine fields between the caller's row order and the handle's: gather
-// (dst[k][i] = src[k][perm[i]], a non-finite value sets the error word) or
-// scatter (dst[k][perm[i]] = src[k][i]).
+// (dst[k][i] = src[k][perm[i]], and zero[k][i] = 0) or scatter (dst[k][perm[i]]
+// = src[k][i]).  A gather writes nothing once k_check_finite has set the error
+// word, so rejected values leave the state as it was.
 struct PermuteArgs {
     const double* src[9];
     double* dst[9];
+    double* zero[3];
     int fields;
 };
-__global__ void k_permute(int n, const int* __restrict__ perm, PermuteArgs f, int scatter, int* err) {
+__global__ void k_permute(int n, const int* __restrict__ perm, PermuteArgs f, int scatter,
+                          const int* __restrict__ err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (!scatter && err[kErrNonFinite]) return;
     const int p = perm[i];
     for (int k = 0; k < f.fields; k++) {
-        if (scatter) {
-            f.dst[k][p] = f.src[k][i];
-        } else {
-            const double v = f.src[k][p];
-            if (!isfinite(v)) dev_flag(err, kErrNonFinite);
-            f.dst[k][i] = v;
-        }
+        if (scatter) f.dst[k][p] = f.src[k][i];
+        else f.dst[k][i] = f.src[k][p];
     }
+    if (!scatter)
+        for (int k = 0; k < 3; k++) f.zero[k][i] = 0.0;
 }
 
 }  // namespace
@@ -912,12 +920,15 @@ NB_API int32_t nb_ens_set_state(nb_ensemble* h, const double* px, const double* 
         f.src[k] = h->d_stage + k * n;
         f.dst[k] = dst[k];
     }
+    f.zero[0] = h->s.ax;
+    f.zero[1] = h->s.ay;
+    f.zero[2] = h->s.az;
     NE_CUDA(h, nb::copy_up(h->io, h->st, seg, 7));
+    nb::k_check_finite<<<std::min(nb::ceil_div(7LL * h->n, 256), 8 * h->sms), 256, 0, h->st>>>(
+        7 * n, h->d_stage, h->scal->err);
     nb::k_permute<<<nb::ceil_div(h->n, 256), 256, 0, h->st>>>(h->n, h->d_perm, f, 0, h->scal->err);
-    NE_CUDA(h, cudaMemsetAsync(h->s.ax, 0, sizeof(double) * h->n, h->st));
-    NE_CUDA(h, cudaMemsetAsync(h->s.ay, 0, sizeof(double) * h->n, h->st));
-    NE_CUDA(h, cudaMemsetAsync(h->s.az, 0, sizeof(double) * h->n, h->st));
     const int r = ens_check(h);
+    if (r == NB_ERR_NONFINITE) return efail(h, r, "non-finite input");
     if (r) return r;
     h->has_state = true;
     h->has_acc = false;
