@@ -85,8 +85,8 @@ k_diag_final(int nblocks, const double* __restrict__ part, int n_items,
 // fills the GPU evenly; one thread per row over all later rows, with a
 // correctly rounded square root and division per pair, left the first rows'
 // blocks running alone.  A whole diagnostics call, before -> now: 2,000
-// bodies 444 -> 57 us, 65,537 bodies 13.39 -> 2.06 ms, 131,072 bodies 29.3 ->
-// 8.2 ms (the FP64 pipe is 71 % busy; 1, 3 and 4 rows per thread were within 5 %).
+// bodies 444 -> 54 us, 65,537 bodies 13.39 -> 2.00 ms, 131,072 bodies 29.3 ->
+// 7.9 ms (1, 3 and 4 rows per thread were within 5 %).
 constexpr int kPeThreads = 256;
 constexpr int kPeRows = 2;                        // rows per thread
 constexpr int kPeTile = kPeThreads * kPeRows;     // rows per item
@@ -130,7 +130,7 @@ k_pe_items(int n, State s, double eps2, int chunk, double* __restrict__ out) {
 #pragma unroll
                 for (int u = 0; u < kPeRows; u++) {
                     const double dx = q.x - xi[u], dy = q.y - yi[u], dz = q.z - zi[u];
-                    acc[u] = fma(q.w, rsqrt_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), acc[u]);
+                    acc[u] = fma(q.w, rsqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), acc[u]);
                 }
             }
         } else {
@@ -140,7 +140,7 @@ k_pe_items(int n, State s, double eps2, int chunk, double* __restrict__ out) {
                 for (int u = 0; u < kPeRows; u++) {
                     if (base + k <= row[u]) continue;
                     const double dx = q.x - xi[u], dy = q.y - yi[u], dz = q.z - zi[u];
-                    acc[u] = fma(q.w, rsqrt_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), acc[u]);
+                    acc[u] = fma(q.w, rsqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), acc[u]);
                 }
             }
         }

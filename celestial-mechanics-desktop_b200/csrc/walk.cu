@@ -1167,7 +1167,7 @@ k_walk_group(WalkArgs a) {
 // monopole only, leaves direct, self skipped, mass-0 nodes skipped.  The
 // acceptance test rounds as compute_force_on_body (barnes_hut_solver.cpp:
 // 230-286) rounds it, so every body meets the reference's cells; their terms
-// are summed in another order and with a 1/sqrt good to FP64 rounding.
+// are summed in another order and with CUDA's rsqrt.
 // Leaves use GravityKernel's shell theorem when `shell`
 // (BarnesHutBackend.cs:410-424).
 //
@@ -1247,7 +1247,7 @@ __global__ void __launch_bounds__(kRefWarps * 32, 4) k_walk_reference(WalkArgs a
                 if (SHELL && R > 0.0 && sqrt(d2) < R) {
                     f = ref_shell(cm.w, R, a.eps2);
                 } else {
-                    const double inv = rsqrt_f64(d2 + a.eps2);
+                    const double inv = rsqrt(d2 + a.eps2);
                     f = cm.w * (inv * inv * inv);
                 }
                 ax = fma(-f, dx, ax);
@@ -1264,7 +1264,7 @@ __global__ void __launch_bounds__(kRefWarps * 32, 4) k_walk_reference(WalkArgs a
                 if (SHELL && R > 0.0 && sqrt(e2) < R) {
                     f = ref_shell(q.w, R, a.eps2);
                 } else {
-                    const double inv = rsqrt_f64(e2 + a.eps2);
+                    const double inv = rsqrt(e2 + a.eps2);
                     f = q.w * (inv * inv * inv);
                 }
                 ax = fma(-f, ex, ax);
