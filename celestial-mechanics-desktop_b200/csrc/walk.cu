@@ -1199,6 +1199,15 @@ __device__ __forceinline__ double ref_shell(double m, double R, double eps2) {
     return __dmul_rn(m, 1.0 / sqrt(den)) / den;
 }
 
+// Coefficient of a point source; a leaf's, with the shell theorem, is multiplied
+// up one factor at a time as GravityKernel does, so that it keeps its bits where
+// inv^3 alone is subnormal (beyond 1e102).
+template <bool SHELL>
+__device__ __forceinline__ double ref_point(double m, double inv, bool leaf) {
+    if (SHELL && leaf) return m * inv * inv * inv;
+    return m * (inv * inv * inv);
+}
+
 template <bool SHELL>
 __global__ void __launch_bounds__(kRefWarps * 32, 4) k_walk_reference(WalkArgs a) {
     __shared__ int2 s_stack[kRefWarps][kRefStack];  // node, body mask
@@ -1246,8 +1255,7 @@ __global__ void __launch_bounds__(kRefWarps * 32, 4) k_walk_reference(WalkArgs a
                 if (SHELL && R > 0.0 && sqrt(d2) < R) {
                     f = ref_shell(cm.w, R, a.eps2);
                 } else {
-                    const double inv = rsqrt(d2 + a.eps2);
-                    f = cm.w * (inv * inv * inv);
+                    f = ref_point<SHELL>(cm.w, rsqrt(d2 + a.eps2), leaf);
                 }
                 ax = fma(-f, dx, ax);
                 ay = fma(-f, dy, ay);
@@ -1274,8 +1282,7 @@ __global__ void __launch_bounds__(kRefWarps * 32, 4) k_walk_reference(WalkArgs a
                 if (SHELL && R > 0.0 && sqrt(e2) < R) {
                     f = ref_shell(q.w, R, a.eps2);
                 } else {
-                    const double inv = rsqrt(e2 + a.eps2);
-                    f = q.w * (inv * inv * inv);
+                    f = ref_point<SHELL>(q.w, rsqrt(e2 + a.eps2), true);
                 }
                 ax = fma(-f, ex, ax);
                 ay = fma(-f, ey, ay);

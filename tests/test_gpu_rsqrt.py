@@ -14,6 +14,7 @@ import pytest
 
 from conftest import PKG_DIR
 from nbody_b200 import MODE_BARNES_HUT_REF, scenarios
+from nbody_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
 
@@ -115,3 +116,15 @@ def test_reference_walk_of_a_pair_at_any_distance(engine, exp):
     want = 3.0 / d / d
     np.testing.assert_allclose(ax, [want, -want], rtol=2.0 ** -49)
     assert not ay.any() and not az.any()
+
+
+@pytest.mark.parametrize("radius", [0.0, 1.0])
+def test_reference_walk_shell_leaf_beyond_the_cube_roots_range(engine, radius):
+    """Heavy bodies so far apart that 1/d^3 is subnormal but m/d^3 is not: the
+    leaf's coefficient is built one factor at a time, each within one unit."""
+    b = _pair(1.7e105, 3e60)
+    b.radius = np.full(2, radius)
+    ax, _, _ = engine.compute_forces(b.px, b.py, b.pz, b.mass, b.active, 0.0,
+                                     MODE_BARNES_HUT_REF | N.FLAG_SHELL_THEOREM, radius=b.radius)
+    want = 3e60 / 1.7e105 / 1.7e105
+    np.testing.assert_allclose(ax, [want, -want], rtol=2.0 ** -49)
