@@ -43,10 +43,14 @@ constexpr size_t kRowAlign = 256;
 // A handle's pinned half.  The forces of 20,011 bodies (0.66 MB up, 0.48 MB
 // down) take 0.48 ms a call, with 256 KB 0.52 and with 1 MB 0.50.
 constexpr size_t kHalfBytes = 512 << 10;
-// The pool takes transfers from these sizes on, where its threads' wake-up is
-// paid for: 7.6 MB up before ten steps of 100,000 bodies 8.7 ms in all against
-// 9.2 plain, 4.8 MB down 0.42 against 0.82.
-constexpr size_t kPoolUp = 4 << 20, kPoolDown = 2 << 20;
+// The pool takes transfers from these sizes on.  Up, the driver's own staging
+// keeps pace with the pool while the arrays come from the caches, and to some
+// 20 MB where they do not (plain / pool, ms, caller's arrays hot: 8 MB 0.44 / 0.92,
+// 16 MB 0.94 / 1.3, 24 MB 1.23 / 1.53, 28 MB 1.6 / 1.5, 48 MB 2.7 / 2.2, 96 MB
+// 8.4 / 3.3; cold: 8 MB 0.7 / 0.9, 16 MB 1.3 / 1.4, 24 MB 2.0 / 1.7, 48 MB 4.3 / 2.4).
+// Down the pool is ahead from 1 MB on (2 MB 0.27 / 0.18, 12 MB 0.97 / 0.43, 96 MB
+// 5.7 / 2.2).
+constexpr size_t kPoolUp = 28 << 20, kPoolDown = 2 << 20;
 // Pinning the slots takes 14 ms, what the plain copy of this much costs more
 // than the pool's: a program that moves less never pays for them.
 constexpr size_t kPoolAfter = 32 << 20;
