@@ -656,9 +656,9 @@ NB_API int32_t nb_create(int32_t capacity, int32_t device, nb_engine** out) {
              })))
             break;
         if ((r = dalloc(h, &h->scal, 1))) break;
-        // a call's arrays up to 256 KB go through the handle's own pinned memory
+        // small calls' arrays go through the handle's own pinned memory
         if (!nb::hostio_init(h->io, device)) {
-            r = fail(h, NB_ERR_CUDA, "pinned memory");
+            r = fail(h, NB_ERR_CUDA, "host memory");
             break;
         }
         static_assert(sizeof(Scal) + sizeof(int) <= nb::kHostExtra, "pinned scalars");

@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -300,15 +301,22 @@ bool hostio_init(HostIO& io, int device) {
             io.pool->spare.pop_back();
         }
     }
-    if (!io.pin && cudaHostAlloc((void**)&io.pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess) {
-        io.pin = nullptr;
-        cudaGetLastError();
-    }
     io.half = kHalfBytes;
+    if (!io.pin && cudaHostAlloc((void**)&io.pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess) {
+        // none to be had: every array takes the plain copy, and the handle's own
+        // bytes are ordinary memory
+        cudaGetLastError();
+        io.half = 0;
+        io.pin = (char*)malloc(kHostExtra);
+    }
     return io.pin != nullptr;
 }
 
 void hostio_free(HostIO& io) {
+    if (io.half == 0) {
+        free(io.pin);
+        io.pin = nullptr;
+    }
     if (io.pin && io.pool) {
         std::lock_guard<std::mutex> lk(g_pools_lock);
         if (io.pool->spare.size() < kMaxSpare) {

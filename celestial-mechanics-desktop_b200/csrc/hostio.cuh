@@ -26,7 +26,8 @@ struct HostIO {
     char* extra() const { return pin + 2 * half; }
 };
 
-// False: no pinned memory.
+// Without pinned memory (half 0) every array takes the plain copy.  False: no
+// memory at all.
 bool hostio_init(HostIO& io, int device);
 void hostio_free(HostIO& io);
 

@@ -101,3 +101,17 @@ def test_uploads_below_the_pools_line_are_plain_copies(host):
     assert c["copies"] >= 12 and c["pinned_copies"] == c["copies"]
     host.lib.t_close(h)
     assert host.counts()["pinned"] == 0
+
+
+def test_a_handle_without_pinned_memory_still_transfers(host):
+    host.lib.t_refuse_pins(1)
+    h = host.open()
+    for total in (96, 60_000, 3 * MB, 40 * MB):
+        for f in (host.up, host.down):
+            assert f(h, total)["pinned_copies"] == 0
+    host.lib.t_refuse_pins(0)
+    other = host.open()
+    assert host.up(other, 60_000)["pinned_copies"] > 0
+    host.lib.t_close(h)
+    host.lib.t_close(other)
+    assert host.counts()["pinned"] == 0
