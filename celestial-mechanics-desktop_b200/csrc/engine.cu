@@ -256,6 +256,7 @@ int check_device(nb_engine* h) {
 }
 
 // Arrays of one transfer; null or empty ones are left out.
+constexpr int kStateRows = 14;  // of the largest, nb_set_state's
 struct Segs {
     nb::CopySeg seg[16];
     int n = 0;
@@ -657,7 +658,7 @@ NB_API int32_t nb_create(int32_t capacity, int32_t device, nb_engine** out) {
             break;
         if ((r = dalloc(h, &h->scal, 1))) break;
         // small calls' arrays go through the handle's own pinned memory
-        if (!nb::hostio_init(h->io, device)) {
+        if (!nb::hostio_init(h->io, device, kStateRows, sizeof(double) * cap)) {
             r = fail(h, NB_ERR_CUDA, "host memory");
             break;
         }

@@ -821,7 +821,10 @@ NB_API int32_t nb_ens_create(int32_t n_systems, const int32_t* sizes, int32_t ds
         nb_ens_destroy(h);
         return r;
     }
-    if (!nb::hostio_init(h->io, device)) {
+    // an ensemble always moves all its bodies: no pinned memory where not even the
+    // 7 arrays of an upload fit it (pinning it takes 1 ms of 5)
+    const size_t row = sizeof(double) * (size_t)h->n;
+    if (!nb::hostio_init(h->io, device, 7 * row <= nb::kHalfBytes ? 9 : 0, row)) {
         nb_ens_destroy(h);
         return NB_ERR_CUDA;
     }

@@ -41,9 +41,6 @@ constexpr size_t kSlotBytes = 1 << 20;
 constexpr size_t kMinChunk = 128 << 10;
 constexpr int kMaxThreads = 7;  // besides the calling one
 constexpr size_t kRowAlign = 256;
-// A handle's pinned half.  The forces of 20,011 bodies (0.66 MB up, 0.48 MB
-// down) take 0.48 ms a call, with 256 KB 0.52 and with 1 MB 0.50.
-constexpr size_t kHalfBytes = 512 << 10;
 // The pool takes transfers from these sizes on.  Up, the driver's own staging
 // keeps pace with the pool while the arrays come from the caches, and to some
 // 20 MB where they do not (plain / pool, ms, caller's arrays hot: 8 MB 0.44 / 0.92,
@@ -55,8 +52,14 @@ constexpr size_t kPoolUp = 28 << 20, kPoolDown = 2 << 20;
 // Pinning the slots takes 14 ms, what the plain copy of this much costs more
 // than the pool's: a program that moves less never pays for them.
 constexpr size_t kPoolAfter = 32 << 20;
-constexpr size_t kPinBytes = 2 * kHalfBytes + kHostExtra;
+constexpr size_t kPage = 4096;
 constexpr size_t kMaxSpare = 8;
+
+// A handle's pinned memory: two halves and kHostExtra bytes.
+struct PinBuf {
+    char* p;
+    size_t half;
+};
 
 struct Chunk {
     char* dst;
@@ -70,7 +73,7 @@ struct CopyPool {
     int device = 0;
     int users = 0;
     char* pin = nullptr;
-    std::vector<char*> spare;   // closed handles' pinned buffers (under g_pools_lock)
+    std::vector<PinBuf> spare;  // closed handles' pinned buffers (under g_pools_lock)
     cudaEvent_t ev[kSlots] = {};
     bool pending[kSlots] = {};  // an upload's copy out of the slot may still run
     std::mutex busy;            // held for a transfer
@@ -203,6 +206,26 @@ struct CopyPool {
 
 namespace {
 
+// Pinned memory as pages of the heap that are registered: 0.4 ms for the 230 KB
+// of a 1,000-body handle, 1 ms for 1 MB, where cudaHostAlloc takes 1.3 to 3 ms
+// for either unless other pinned memory is about (ms to create a handle for
+// 1,000 bodies: 4.2 without pinned memory, 4.9 so, 6.5 that way).
+char* pin(size_t bytes) {
+    char* p = (char*)aligned_alloc(kPage, (bytes + kPage - 1) / kPage * kPage);
+    if (p && cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) {
+        cudaGetLastError();
+        free(p);
+        p = nullptr;
+    }
+    return p;
+}
+
+void unpin(char* p) {
+    if (!p) return;
+    cudaHostUnregister(p);
+    free(p);
+}
+
 std::mutex g_pools_lock;
 std::vector<CopyPool*> g_pools;
 
@@ -218,7 +241,7 @@ void pool_destroy(CopyPool* p) {
             if (p->pending[k]) cudaEventSynchronize(p->ev[k]);
             cudaEventDestroy(p->ev[k]);
         }
-    for (char* b : p->spare) cudaFreeHost(b);
+    for (const PinBuf& b : p->spare) unpin(b.p);
     if (p->pin) cudaFreeHost(p->pin);
     delete p;
 }
@@ -288,24 +311,29 @@ size_t packed_bytes(const CopySeg* seg, int n) {
 
 }  // namespace
 
-bool hostio_init(HostIO& io, int device) {
+bool hostio_init(HostIO& io, int device, int rows, size_t row_bytes) {
     try {
         io.pool = pool_acquire(device);
     } catch (...) {
         io.pool = nullptr;
     }
-    if (io.pool) {
+    const size_t all = (rows * padded(row_bytes) + kPage - 1) / kPage * kPage;
+    io.half = std::min(kHalfBytes, all);
+    if (io.pool && io.half) {
         std::lock_guard<std::mutex> lk(g_pools_lock);
-        if (!io.pool->spare.empty()) {
-            io.pin = io.pool->spare.back();
-            io.pool->spare.pop_back();
+        auto& spare = io.pool->spare;
+        const auto fit = std::find_if(spare.begin(), spare.end(),
+                                      [&](const PinBuf& b) { return b.half >= io.half; });
+        if (fit != spare.end()) {
+            io.pin = fit->p;
+            io.half = fit->half;
+            spare.erase(fit);
         }
     }
-    io.half = kHalfBytes;
-    if (!io.pin && cudaHostAlloc((void**)&io.pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess) {
-        // none to be had: every array takes the plain copy, and the handle's own
-        // bytes are ordinary memory
-        cudaGetLastError();
+    if (!io.pin && io.half) io.pin = pin(2 * io.half + kHostExtra);
+    if (!io.pin) {
+        // none wanted or none to be had: every array takes the plain copy, and
+        // the handle's own bytes are ordinary memory
         io.half = 0;
         io.pin = (char*)malloc(kHostExtra);
     }
@@ -319,12 +347,13 @@ void hostio_free(HostIO& io) {
     }
     if (io.pin && io.pool) {
         std::lock_guard<std::mutex> lk(g_pools_lock);
-        if (io.pool->spare.size() < kMaxSpare) {
-            io.pool->spare.push_back(io.pin);  // capacity was reserved
+        auto& spare = io.pool->spare;
+        if (spare.size() < kMaxSpare) {
+            spare.push_back({io.pin, io.half});  // capacity was reserved
             io.pin = nullptr;
         }
     }
-    if (io.pin) cudaFreeHost(io.pin);
+    unpin(io.pin);
     if (io.pool) pool_release(io.pool);
     io = HostIO();
 }

@@ -86,9 +86,9 @@ cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size
 
 // ---- for the test --------------------------------------------------------
 #define API __attribute__((visibility("default")))
-API void* t_open() {
+API void* t_open(int rows, size_t bytes) {
     nb::HostIO* io = new nb::HostIO();
-    if (!nb::hostio_init(*io, 0)) {
+    if (!nb::hostio_init(*io, 0, rows, bytes)) {
         nb::hostio_free(*io);
         delete io;
         return nullptr;

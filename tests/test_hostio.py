@@ -35,14 +35,14 @@ class Host:
         own = tmp_path / "own.so"  # a path of its own: dlopen shares by path
         shutil.copy(so, own)
         self.lib = lib = C.CDLL(str(own))
-        lib.t_open.restype = C.c_void_p
+        lib.t_open.restype, lib.t_open.argtypes = C.c_void_p, [C.c_int, C.c_size_t]
         lib.t_close.argtypes = [C.c_void_p]
         for f in (lib.t_up, lib.t_down):
             f.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p),
                           C.c_size_t]
 
-    def open(self):
-        h = self.lib.t_open()
+    def open(self, row_bytes=8 * MB, rows=14):
+        h = self.lib.t_open(rows, row_bytes)
         assert h
         return h
 
@@ -114,4 +114,46 @@ def test_a_handle_without_pinned_memory_still_transfers(host):
     assert host.up(other, 60_000)["pinned_copies"] > 0
     host.lib.t_close(h)
     host.lib.t_close(other)
+    assert host.counts()["pinned"] == 0
+
+
+@pytest.mark.parametrize("n", [1, 64, 1000, 4681, 4700, 1 << 20])
+def test_a_handle_pins_what_its_largest_transfer_needs(host, n):
+    """Two halves (up, down) of 14 arrays of n doubles, in whole pages and at
+    most 512 KB each, and 4 KB; the largest transfer is one that fits."""
+    h = host.open(8 * n)
+    rows = -(-8 * n // 256) * 256 * 14
+    half = min(512 << 10, -(-rows // 4096) * 4096)
+    assert host.counts()["pinned"] == 2 * half + 4096
+    for f in (host.up, host.down):
+        c = f(h, 14 * 8 * n, rows=14)
+        if rows <= half:
+            assert c["pinned_copies"] == c["copies"] == 14
+    host.lib.t_close(h)
+    assert host.counts()["pinned"] == 0
+
+
+def test_a_handle_that_wants_no_pinned_memory_pins_none(host):
+    h = host.open(8 * 1000, rows=0)
+    assert host.counts()["pins"] == 0
+    assert host.up(h, 9000)["pinned_copies"] == host.down(h, 9000)["pinned_copies"] == 0
+    host.lib.t_close(h)
+
+
+def test_a_closed_handles_pinned_memory_goes_to_the_next_that_fits(host):
+    keep = host.open(8 * 64)
+    small, large = host.open(8 * 500), host.open(8 * 100_000)
+    pins = host.counts()["pins"]
+    host.lib.t_close(small)
+    host.lib.t_close(large)
+    again = host.open(8 * 100_000)  # the small one's is too small for it
+    assert host.counts()["pins"] == pins
+    host.up(again, 400_000)
+    host.down(again, 400_000)
+    tiny = host.open(8 * 400)
+    assert host.counts()["pins"] == pins
+    many = [host.open(8 * 300) for _ in range(12)]
+    for h in (again, tiny, *many):
+        host.lib.t_close(h)
+    host.lib.t_close(keep)
     assert host.counts()["pinned"] == 0
