@@ -22,6 +22,8 @@
 // as long as the rest of a small handle).
 #include "hostio.cuh"
 
+#include <sched.h>
+
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
@@ -39,7 +41,8 @@ namespace {
 constexpr int kSlots = 16;
 constexpr size_t kSlotBytes = 1 << 20;
 constexpr size_t kMinChunk = 128 << 10;
-constexpr int kMaxThreads = 7;  // besides the calling one
+constexpr int kMaxThreads = 7;  // besides the calling one, and of half the CPUs
+constexpr int kMinThreads = 2;
 constexpr size_t kRowAlign = 256;
 // The pool takes transfers from these sizes on.  Up, the driver's own staging
 // keeps pace with the pool while the arrays come from the caches, and to some
@@ -68,6 +71,13 @@ struct Chunk {
 };
 
 }  // namespace
+
+// CPUs this process may run on.
+static int cpus_here() {
+    cpu_set_t set;
+    if (sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
+    return (int)std::thread::hardware_concurrency();
+}
 
 struct CopyPool {
     int device = 0;
@@ -149,6 +159,8 @@ struct CopyPool {
     // held).  A pool of one or two threads moves no more than the plain copy
     // does: false then, and where there is no pinned memory to be had.
     bool ready(size_t total) {
+        const int want = std::min(kMaxThreads, cpus_here() / 2 - 1);
+        if (want < kMinThreads) return false;
         if (!made) {
             moved += total;
             if (moved < kPoolAfter) return false;
@@ -161,16 +173,14 @@ struct CopyPool {
             for (int k = 0; ok && k < kSlots; k++)
                 ok = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming) == cudaSuccess;
             cudaThreadExchangeStreamCaptureMode(&mode);
-            const int cpus = (int)std::thread::hardware_concurrency();
             try {
-                for (int k = 0; ok && k < std::min(kMaxThreads, cpus / 2 - 1); k++)
-                    threads.emplace_back([this] { loop(); });
+                for (int k = 0; ok && k < want; k++) threads.emplace_back([this] { loop(); });
             } catch (...) {
                 // fewer threads, or none: the calling thread does the rest
             }
             if (!ok) cudaGetLastError();
         }
-        return threads.size() >= 2;
+        return (int)threads.size() >= kMinThreads;
     }
 
     // The whole transfer, with `busy` held.  Returns when every host array has

@@ -120,5 +120,4 @@ API void t_counts(size_t* out) {
     memcpy(out, c, sizeof(c));
 }
 API void t_refuse_pins(int on) { g_refuse_pins = on; }
-API int t_cpus() { return (int)std::thread::hardware_concurrency(); }
 }

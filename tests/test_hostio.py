@@ -3,6 +3,7 @@ on the CPU, over a runtime of plain memory that counts pins and copies."""
 from __future__ import annotations
 
 import ctypes as C
+import multiprocessing
 import os
 import shutil
 import subprocess
@@ -86,7 +87,10 @@ def host(built, tmp_path):
     return Host(built, tmp_path)
 
 
-@pytest.mark.skipif(len(os.sched_getaffinity(0)) < 6, reason="too few CPUs for the pool")
+POOL = pytest.mark.skipif(len(os.sched_getaffinity(0)) < 6, reason="too few CPUs for the pool")
+
+
+@POOL
 def test_uploads_below_the_pools_line_are_plain_copies(host):
     """Up to 28 MB the plain copy of an upload is as fast as the pool or
     faster (12 MB 0.56 against 1.24 ms); downloads go by the pool from 2 MB."""
@@ -157,3 +161,24 @@ def test_a_closed_handles_pinned_memory_goes_to_the_next_that_fits(host):
         host.lib.t_close(h)
     host.lib.t_close(keep)
     assert host.counts()["pinned"] == 0
+
+
+def _on_few_cpus(so, path, cpus):
+    os.sched_setaffinity(0, sorted(os.sched_getaffinity(0))[:cpus])
+    host = Host(so, path)
+    h = host.open(8 * 64)
+    own = host.counts()["pinned"]
+    host.warm(h)
+    host.up(h, 60 * MB)
+    assert host.counts()["pinned"] == own
+    host.lib.t_close(h)
+
+
+@pytest.mark.parametrize("cpus", [1, 5])
+def test_too_few_cpus_for_the_pool_pin_nothing_for_it(built, tmp_path, cpus):
+    """A pool of fewer than two threads is never used, so its slots are not pinned."""
+    p = multiprocessing.get_context("spawn").Process(target=_on_few_cpus,
+                                                     args=(built, tmp_path, cpus))
+    p.start()
+    p.join(120)
+    assert p.exitcode == 0
