@@ -23,8 +23,9 @@ def built(tmp_path_factory):
     if not shutil.which("g++") or not (CUDA_INCLUDE / "cuda_runtime.h").exists():
         pytest.skip("no g++ or no CUDA headers")
     so = tmp_path_factory.mktemp("hostio") / "hostio_fake.so"
-    subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-shared", "-fPIC", "-pthread", "-I",
-                    str(PKG_DIR / "csrc"), "-I", str(CUDA_INCLUDE), "-x", "c++", "-o", str(so),
+    subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-shared", "-fPIC", "-pthread",
+                    "-Wl,-Bsymbolic",  # its own runtime, whatever else is loaded
+                    "-I", str(PKG_DIR / "csrc"), "-I", str(CUDA_INCLUDE), "-x", "c++", "-o", str(so),
                     str(Path(__file__).parent / "hostio_fake.cpp")], check=True)
     return so
 
