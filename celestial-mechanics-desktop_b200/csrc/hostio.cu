@@ -10,11 +10,11 @@
 //     per call.
 //   * A large one is cut into chunks that a pool of threads moves through a
 //     ring of pinned slots, so the host copies run side by side and overlap
-//     the bus.  There is one pool per device; its slots (kSlots MB pinned) and
-//     threads (at most kMaxThreads) come when kPoolAfter bytes have gone the
-//     plain way, and go with the device's last handle.  A transfer holds the
-//     pool for itself; when another thread's transfer has it, the plain copy
-//     is used instead, so handles never wait for each other.
+//     the bus.  There is one pool per device; its threads (at most kMaxThreads)
+//     and the first of its slots (up to kSlots MB pinned) come when kPoolAfter
+//     bytes have gone the plain way, and go with the device's last handle.  A
+//     transfer holds the pool for itself; when another thread's transfer has it,
+//     the plain copy is used instead, so handles never wait for each other.
 // Before -> now: forces of 2^20 bodies 11.8 -> 8.4 ms a call (5.4 of them on
 // the GPU), of 1,000 bodies 136 -> 82 us, a read-back of 2^20 bodies' state
 // 46 -> 6.3 ms, of an ensemble's 804,337 bodies 25 -> 5.2 ms.  A closed
@@ -52,9 +52,12 @@ constexpr size_t kRowAlign = 256;
 // Down the pool is ahead from 1 MB on (2 MB 0.27 / 0.18, 12 MB 0.97 / 0.43, 96 MB
 // 5.7 / 2.2).
 constexpr size_t kPoolUp = 28 << 20, kPoolDown = 2 << 20;
-// Pinning the slots takes 14 ms, what the plain copy of this much costs more
-// than the pool's: a program that moves less never pays for them.
+// The slots come once a program has moved this much by plain copies: one that
+// moves less never pays for them.  They come a few at a time, so that no call is
+// held up by more than 2 to 3 ms, and the six after it by 1.3 (all 16 MB at once
+// took 7 to 10, and up to 20 on another host).
 constexpr size_t kPoolAfter = 32 << 20;
+constexpr int kFirstSlots = 4, kMoreSlots = 2;
 constexpr size_t kPage = 4096;
 constexpr size_t kMaxSpare = 8;
 
@@ -70,20 +73,42 @@ struct Chunk {
     size_t bytes;
 };
 
-}  // namespace
+// Pinned memory as pages of the heap that are registered: 0.4 ms for the 230 KB
+// of a 1,000-body handle, 1 ms for 1 MB, where cudaHostAlloc takes 1.3 to 3 ms
+// for either unless other pinned memory is about (ms to create a handle for
+// 1,000 bodies: 4.2 without pinned memory, 4.9 so, 6.5 that way).
+char* pin(size_t bytes) {
+    char* p = (char*)aligned_alloc(kPage, (bytes + kPage - 1) / kPage * kPage);
+    if (p && cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) {
+        cudaGetLastError();
+        free(p);
+        p = nullptr;
+    }
+    return p;
+}
+
+void unpin(char* p) {
+    if (!p) return;
+    cudaHostUnregister(p);
+    free(p);
+}
 
 // CPUs this process may run on.
-static int cpus_here() {
+int cpus_here() {
     cpu_set_t set;
     if (sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
     return (int)std::thread::hardware_concurrency();
 }
 
+}  // namespace
+
 struct CopyPool {
     int device = 0;
     int users = 0;
-    char* pin = nullptr;
     std::vector<PinBuf> spare;  // closed handles' pinned buffers (under g_pools_lock)
+    int slots = 0;              // that are there (under busy)
+    bool full = false;          // no more to be had (under busy)
+    char* buf[kSlots] = {};
     cudaEvent_t ev[kSlots] = {};
     bool pending[kSlots] = {};  // an upload's copy out of the slot may still run
     std::mutex busy;            // held for a transfer
@@ -102,18 +127,17 @@ struct CopyPool {
     bool open = false;  // the job still takes threads
     int inside = 0;     // threads at work on it
     bool stop = false;
-    bool made = false;  // slots, events and threads (under busy)
-    size_t moved = 0;   // bytes that went the plain way before that (under busy)
+    size_t moved = 0;   // bytes that went the plain way before the slots (under busy)
 
-    // Chunk c goes through slot c % kSlots when the slot's earlier chunks have
+    // Chunk c goes through slot c % slots when the slot's earlier chunks have
     // left it (up: its copy was enqueued, and its event says when it ended;
     // down: its data is in the host array).
     void work() {
         for (;;) {
             const int c = next.fetch_add(1);
             if (c >= (int)chunks.size()) return;
-            const int slot = c % kSlots, my_turn = c / kSlots;
-            char* buf = pin + (size_t)slot * kSlotBytes;
+            const int slot = c % slots, my_turn = c / slots;
+            char* const own = buf[slot];
             while (turn[slot].load(std::memory_order_acquire) != my_turn) std::this_thread::yield();
             cudaError_t e = cudaSuccess;
             if (pending[slot]) {
@@ -122,17 +146,17 @@ struct CopyPool {
             }
             const Chunk& k = chunks[c];
             if (up) {
-                std::memcpy(buf, k.src, k.bytes);
+                std::memcpy(own, k.src, k.bytes);
                 if (e == cudaSuccess)
-                    e = cudaMemcpyAsync(k.dst, buf, k.bytes, cudaMemcpyHostToDevice, st);
+                    e = cudaMemcpyAsync(k.dst, own, k.bytes, cudaMemcpyHostToDevice, st);
                 if (e == cudaSuccess) e = cudaEventRecord(ev[slot], st);
                 pending[slot] = true;
             } else {
                 if (e == cudaSuccess)
-                    e = cudaMemcpyAsync(buf, k.src, k.bytes, cudaMemcpyDeviceToHost, st);
+                    e = cudaMemcpyAsync(own, k.src, k.bytes, cudaMemcpyDeviceToHost, st);
                 if (e == cudaSuccess) e = cudaEventRecord(ev[slot], st);
                 if (e == cudaSuccess) e = cudaEventSynchronize(ev[slot]);
-                if (e == cudaSuccess) std::memcpy(k.dst, buf, k.bytes);
+                if (e == cudaSuccess) std::memcpy(k.dst, own, k.bytes);
             }
             if (e != cudaSuccess) failed.store((int)e);
             turn[slot].store(my_turn + 1, std::memory_order_release);
@@ -144,7 +168,8 @@ struct CopyPool {
         unsigned long long seen = 0;
         std::unique_lock<std::mutex> lk(m);
         for (;;) {
-            wake.wait(lk, [&] { return stop || (open && job != seen); });
+            // (more threads than slots would only wait for one another)
+            wake.wait(lk, [&] { return stop || (open && job != seen && inside < slots - 1); });
             if (stop) return;
             seen = job;
             inside++;
@@ -155,30 +180,43 @@ struct CopyPool {
         }
     }
 
-    // Slots, events and threads, once kPoolAfter bytes have gone without (busy
-    // held).  A pool of one or two threads moves no more than the plain copy
-    // does: false then, and where there is no pinned memory to be had.
+    // `count` more slots (busy held).
+    void grow(int count) {
+        // another thread of the program may be capturing a graph
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        for (; count > 0 && slots < kSlots && !full; count--) {
+            buf[slots] = pin(kSlotBytes);
+            if (buf[slots] &&
+                cudaEventCreateWithFlags(&ev[slots], cudaEventDisableTiming) == cudaSuccess) {
+                slots++;
+            } else {
+                cudaGetLastError();
+                unpin(buf[slots]);
+                buf[slots] = nullptr;
+                full = true;
+            }
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+
+    // Slots and threads, once kPoolAfter bytes have gone without (busy held).  A
+    // pool of one or two threads moves no more than the plain copy does: false
+    // then, and where there is no pinned memory to be had.
     bool ready(size_t total) {
         const int want = std::min(kMaxThreads, cpus_here() / 2 - 1);
         if (want < kMinThreads) return false;
-        if (!made) {
+        if (slots == 0) {
             moved += total;
             if (moved < kPoolAfter) return false;
-            made = true;
-            // another thread of the program may be capturing a graph
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            bool ok = cudaHostAlloc((void**)&pin, kSlots * kSlotBytes, cudaHostAllocDefault) ==
-                      cudaSuccess;
-            for (int k = 0; ok && k < kSlots; k++)
-                ok = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming) == cudaSuccess;
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            try {
-                for (int k = 0; ok && k < want; k++) threads.emplace_back([this] { loop(); });
-            } catch (...) {
-                // fewer threads, or none: the calling thread does the rest
-            }
-            if (!ok) cudaGetLastError();
+        }
+        grow(slots ? kMoreSlots : kFirstSlots);
+        if (slots < kFirstSlots) return false;
+        try {
+            if (threads.empty())
+                for (int k = 0; k < want; k++) threads.emplace_back([this] { loop(); });
+        } catch (...) {
+            // fewer threads, or none: the calling thread does the rest
         }
         return (int)threads.size() >= kMinThreads;
     }
@@ -186,7 +224,7 @@ struct CopyPool {
     // The whole transfer, with `busy` held.  Returns when every host array has
     // been read or written.
     cudaError_t run(bool upward, cudaStream_t stream, const CopySeg* seg, int n, size_t total) {
-        const size_t parts = 2 * (threads.size() + 1);
+        const size_t parts = 2 * std::min(threads.size() + 1, (size_t)slots);
         const size_t want = std::min(kSlotBytes, std::max(kMinChunk, total / parts));
         const size_t chunk = (want + 4095) / 4096 * 4096;
         chunks.clear();
@@ -216,26 +254,6 @@ struct CopyPool {
 
 namespace {
 
-// Pinned memory as pages of the heap that are registered: 0.4 ms for the 230 KB
-// of a 1,000-body handle, 1 ms for 1 MB, where cudaHostAlloc takes 1.3 to 3 ms
-// for either unless other pinned memory is about (ms to create a handle for
-// 1,000 bodies: 4.2 without pinned memory, 4.9 so, 6.5 that way).
-char* pin(size_t bytes) {
-    char* p = (char*)aligned_alloc(kPage, (bytes + kPage - 1) / kPage * kPage);
-    if (p && cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) {
-        cudaGetLastError();
-        free(p);
-        p = nullptr;
-    }
-    return p;
-}
-
-void unpin(char* p) {
-    if (!p) return;
-    cudaHostUnregister(p);
-    free(p);
-}
-
 std::mutex g_pools_lock;
 std::vector<CopyPool*> g_pools;
 
@@ -252,7 +270,7 @@ void pool_destroy(CopyPool* p) {
             cudaEventDestroy(p->ev[k]);
         }
     for (const PinBuf& b : p->spare) unpin(b.p);
-    if (p->pin) cudaFreeHost(p->pin);
+    for (char* b : p->buf) unpin(b);
     delete p;
 }
 

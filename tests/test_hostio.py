@@ -183,3 +183,35 @@ def test_too_few_cpus_for_the_pool_pin_nothing_for_it(built, tmp_path, cpus):
     p.start()
     p.join(120)
     assert p.exitcode == 0
+
+
+@POOL
+@pytest.mark.parametrize("mb", [3, 40])
+def test_the_pools_slots_come_a_few_at_a_time(host, mb):
+    """No call pins more than the first 4 MB, and the pool works from then on,
+    while it grows to 16 MB."""
+    h = host.open(8 * 64)
+    own = host.counts()["pinned"]
+    pinned = []
+    for _ in range(24):
+        c = host.down(h, mb * MB)
+        pinned.append(c["pinned"])
+        assert (c["pinned_copies"] > 0) == (sum(pinned) > 0)
+    first = pinned.index(4 * MB)
+    assert first * mb < 32 <= (first + 1) * mb
+    assert pinned[first + 1:first + 8] == [2 * MB] * 6 + [0]
+    host.up(h, 60 * MB)
+    assert host.counts()["pinned"] == own + 16 * MB
+    host.lib.t_close(h)
+    assert host.counts()["pinned"] == 0
+
+
+@POOL
+def test_a_pool_that_gets_no_slots_leaves_the_plain_copy(host):
+    h = host.open(8 * 64)
+    host.lib.t_refuse_pins(1)
+    host.warm(h)
+    assert host.down(h, 8 * MB)["pinned_copies"] == 0
+    host.lib.t_refuse_pins(0)
+    assert host.down(h, 8 * MB)["pinned_copies"] == 0
+    host.lib.t_close(h)
