@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "direct.cuh"
+#include "tree.cuh"
 
 namespace nb {
 
@@ -770,10 +771,13 @@ void direct_fp32(cudaStream_t st, int n, const double4* sbody, const float* srad
     // Chunks: from each chunk on the j-tiles start anew, so the chunk length
     // decides how the FP32 sums round, and it keeps to this rule: items of
     // kD32Ref targets make at least 4 waves on one block per SM where 4096
-    // sources per chunk and the handle's 290 bytes per body allow it, and among
-    // those counts the fewest chunks within 0.5 % of the fullest last wave.
+    // sources per chunk and some 290 bytes of `part` per body allow it, and among
+    // those counts the fewest chunks within 0.5 % of the fullest last wave.  (The
+    // byte count keeps the chunks where they were when the tree's memory, which
+    // `part` is, had that size; it never exceeds what is there.)
     const int tiles = ceil_div(n, kD32Ref);
-    const long long room = 290LL * capacity + (capacity / 1024 + 2) * 4 + 1328;
+    const long long room = std::min<long long>(
+        290LL * capacity + (capacity / 1024 + 2) * 4 + 1328, (long long)tree_bytes(capacity));
     const long long cmax =
         std::max<long long>(1, std::min<long long>(std::max(1, ceil_div(n, 4096)), room / (24LL * n)));
     const long long cmin = std::min<long long>(cmax, std::max(1, ceil_div(4LL * sms, tiles)));
