@@ -468,7 +468,7 @@ __global__ void k_direct_reduce(int n, int chunks, const double* __restrict__ pa
 // overlap.  A term that is not added (the body itself, an inactive source) is
 // stored as +0, whose subtraction changes no bit.  The chain bounds a small
 // system (1000 dependent additions), the square root and division a large
-// one; the two buffers are 2 x 25 KB at TI = 8, so two blocks share an SM.
+// one; the two buffers are 2 x 25 KB at TI = 8, and three blocks share an SM.
 // Two phases of a tile behind one another, 256 threads for both, took 51.2 us
 // for 1,000 bodies, 731 us for 8,192 and 3.47 ms for 20,000; now 21.5, 273 and
 // 1,424 us (call times on the stream; 10, 53 and 60 % of the FP64 rate by some

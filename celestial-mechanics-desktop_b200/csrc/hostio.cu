@@ -15,11 +15,10 @@
 //     bytes have gone the plain way, and go with the device's last handle.  A
 //     transfer holds the pool for itself; when another thread's transfer has it,
 //     the plain copy is used instead, so handles never wait for each other.
-// Before -> now: forces of 2^20 bodies 11.8 -> 8.4 ms a call (5.4 of them on
-// the GPU), of 1,000 bodies 136 -> 82 us, a read-back of 2^20 bodies' state
-// 46 -> 6.3 ms, of an ensemble's 804,337 bodies 25 -> 5.2 ms.  A closed
-// handle's pinned buffer waits for the next handle (pinning 1 MB takes 1 to 4 ms,
-// as long as the rest of a small handle).
+// Before -> now, by these transfers: forces of 2^20 bodies 11.8 -> 8.7 ms a call
+// (5.4 of them on the GPU) and of 1,000 bodies 136 -> 82 us; read-backs into new
+// arrays, of 2^20 bodies' state 35 -> 2.3 ms and of an ensemble's 804,337 bodies
+// 19 -> 1.5 ms.  A closed handle's pinned buffer waits for the next handle.
 #include "hostio.cuh"
 
 #include <sched.h>

@@ -31,8 +31,10 @@ namespace nb {
 
 constexpr int kMarkThreads = 256;
 // Binary nodes per thread of the marking and numbering kernels: 1, since a
-// node's climb is a chain of dependent loads (20,011 bodies: tree stage 107 ->
-// 85 us against 4), 4 above 2^20 bodies, where the blocks' sums get many.
+// node's climb is a chain of dependent loads, and 4 above 2^20 bodies, where the
+// blocks' sums would get more than kMarkScanBlocks (tree stage, us, 1 / 4 per
+// thread: 65,536 bodies 83 / 95, 262,144 99 / 112, 750,000 173 / 175, 2^20 210 /
+// 210, 1,300,000 246 / 237, 2^21 340 / 323, 2^22 598 / 550).
 constexpr int kMarkItems = 4;
 constexpr int kMarkManyNodes = 1 << 20;
 // blocks whose sums a block of the numbering kernel adds up itself; more are
