@@ -759,8 +759,14 @@ cudaError_t direct_fp64_steps(cudaStream_t st, Fp64Args a, bool shell, int order
     return e;
 }
 
-// Bodies up to which k_direct_fp32_rows is the faster one.
-constexpr int kD32RowsMax = 200000;
+// Fullness of the tiles' waves (items over the slots of their whole waves) from
+// which k_direct_fp32 is the faster one: its items run 2.5 % faster than the
+// rows', which end evenly whatever their number.  tile / row kernel, ms: 50,000
+// bodies (0.88 full) 1.13 / 1.07, 100,003 0.81 full 4.80 / 3.98 and 0.99 full
+// (a roomier handle: more chunks) 3.95 / 3.97, 150,000 0.96 full 8.98 / 8.87 and
+// 0.997 full 8.64 / 8.85, 262,144 (0.994) 26.3 / 27.0, 350,000 0.93 full 50.0 /
+// 48.4 and 0.997 full 46.5 / 47.8.
+constexpr double kD32TileFill = 0.975;
 
 void direct_fp32(cudaStream_t st, int n, const double4* sbody, const float* srad,
                  const uint32_t* sidx, double eps, bool shell, double* ax, double* ay,
@@ -800,11 +806,8 @@ void direct_fp32(cudaStream_t st, int n, const double4* sbody, const float* srad
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
         return std::min(items, sms * std::max(1, per_sm));
     };
-    // items of 2560 targets only where they are many waves: k_direct_fp32 against
-    // the rows 301 / 60 us at 2,000 bodies, 590 / 220 at 20,000, 4,820 / 3,980 at
-    // 100,003 (480 items are 3.2 waves and took four), 12.92 / 12.77 ms at
-    // 180,000, 26.3 / 27.0 at 262,144; shells (rows only now) 38.4 / 34.6 there
-    if (!shell && n > kD32RowsMax) {
+    // shells have the row kernel only (262,144: 38.4 by tiles / 34.6 ms)
+    if (!shell && fill(chunks) >= kD32TileFill) {
         const auto k = eps2 > 0.f ? k_direct_fp32<false> : k_direct_fp32<true>;
         const int items = tiles * nchunks;
         k<<<grid(k, kD32Threads, kD32Smem, items), kD32Threads, kD32Smem, st>>>(
