@@ -1544,11 +1544,17 @@ void walk_group(cudaStream_t st, const WalkConfig& cfg, WalkArgs a, bool quad, b
     const bool g64 = a.group_size == 64 && a.group_span >= 64 && quad && !shell && !pot &&
                      (mac != kMacGeometric || shape == 0);
     // Helping pays while the grid's warps have at most some three groups each:
-    // plain -> helping at theta 0.5, 64-body groups, 20,011 bodies 455 -> 207 us,
-    // 100,003 730 -> 590, 400,000 2,080 -> 2,020; 2^20 (seven groups per warp)
-    // 5,370 -> 5,420, and 576,000 bodies in 137 systems lose 2 %.  The forces are
-    // the same bits either way.
-    auto help_pays = [&](int warps, int size) { return a.n <= 3LL * warps * size; };
+    // plain -> helping at theta 0.5, 64-body groups, 20,011 bodies 432 -> 180 us,
+    // 100,003 637 -> 575, 400,000 2,137 -> 2,094; 2^20 (seven groups per warp)
+    // 5,370 -> 5,420, and 576,000 bodies in 137 systems lose 2 %.  32-body groups
+    // gain to two groups per warp and are even at three, but there a disk of
+    // 262,145 bodies with shells still gains (805 -> 640).  Without quadrupoles a
+    // list takes half as long to evaluate, and it ends at one and a half (20,011
+    // bodies 275 -> 173, 150,000 685 -> 670, 180,000 782 -> 798, 300,000 1,253 ->
+    // 1,279).  The forces are the same bits either way.
+    auto help_pays = [&](int warps, int size) {
+        return 2LL * a.n <= (quad ? 6LL : 3LL) * warps * size;
+    };
     find_groups(st, a.t, a.sbody, a.n, a.groups, a.n_groups, a.pack, a.group_span,
                 g64 ? 64 : 32, a.zeroed);
     if (!a.zeroed) cudaMemsetAsync(a.group_ctr, 0, sizeof(unsigned), st);
