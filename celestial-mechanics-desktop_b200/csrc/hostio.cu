@@ -22,6 +22,7 @@
 #include "hostio.cuh"
 
 #include <sched.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <atomic>
@@ -72,25 +73,32 @@ struct Chunk {
     size_t bytes;
 };
 
-// Pinned memory as pages of the heap that are registered: 0.4 ms for the 230 KB
+// Pinned memory as ordinary pages that are registered: 0.4 ms for the 230 KB
 // of a 1,000-body handle, 1 ms for 1 MB, where cudaHostAlloc takes 1.3 to 3 ms
 // for either unless other pinned memory is about (ms to create a handle for
-// 1,000 bodies: 4.2 without pinned memory, 4.9 so, 6.5 that way).
+// 1,000 bodies: 4.2 without pinned memory, 4.9 so, 6.5 that way).  A child process
+// does not inherit them: a fork would otherwise have the parent write to copies
+// of the pages while the device keeps to the old ones, where the kernel does
+// not look after registered pages itself.
 char* pin(size_t bytes) {
-    char* p = (char*)aligned_alloc(kPage, (bytes + kPage - 1) / kPage * kPage);
-    if (p && cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) {
+    void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (p == MAP_FAILED) return nullptr;
+    if (madvise(p, bytes, MADV_DONTFORK) != 0 ||
+        cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) {
         cudaGetLastError();
-        free(p);
-        p = nullptr;
+        munmap(p, bytes);
+        return nullptr;
     }
-    return p;
+    return (char*)p;
 }
 
-void unpin(char* p) {
+void unpin(char* p, size_t bytes) {
     if (!p) return;
     cudaHostUnregister(p);
-    free(p);
+    munmap(p, bytes);
 }
+
+size_t pin_bytes(size_t half) { return 2 * half + kHostExtra; }
 
 // CPUs this process may run on.
 int cpus_here() {
@@ -191,7 +199,7 @@ struct CopyPool {
                 slots++;
             } else {
                 cudaGetLastError();
-                unpin(buf[slots]);
+                unpin(buf[slots], kSlotBytes);
                 buf[slots] = nullptr;
                 full = true;
             }
@@ -268,8 +276,8 @@ void pool_destroy(CopyPool* p) {
             if (p->pending[k]) cudaEventSynchronize(p->ev[k]);
             cudaEventDestroy(p->ev[k]);
         }
-    for (const PinBuf& b : p->spare) unpin(b.p);
-    for (char* b : p->buf) unpin(b);
+    for (const PinBuf& b : p->spare) unpin(b.p, pin_bytes(b.half));
+    for (char* b : p->buf) unpin(b, kSlotBytes);
     delete p;
 }
 
@@ -357,7 +365,7 @@ bool hostio_init(HostIO& io, int device, int rows, size_t row_bytes) {
             spare.erase(fit);
         }
     }
-    if (!io.pin && io.half) io.pin = pin(2 * io.half + kHostExtra);
+    if (!io.pin && io.half) io.pin = pin(pin_bytes(io.half));
     if (!io.pin) {
         // none wanted or none to be had: every array takes the plain copy, and
         // the handle's own bytes are ordinary memory
@@ -380,7 +388,7 @@ void hostio_free(HostIO& io) {
             io.pin = nullptr;
         }
     }
-    unpin(io.pin);
+    unpin(io.pin, pin_bytes(io.half));
     if (io.pool) pool_release(io.pool);
     io = HostIO();
 }

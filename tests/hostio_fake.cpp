@@ -119,5 +119,11 @@ API void t_counts(size_t* out) {
     const size_t c[5] = {g_pinned_now, g_pinned_sum, g_pins, g_copies, g_pinned_copies};
     memcpy(out, c, sizeof(c));
 }
+// The start of some pinned memory, and its bytes.
+API void t_some_pinned(size_t* out) {
+    std::lock_guard<std::mutex> lk(g);
+    out[0] = (size_t)g_pinned.begin()->first;
+    out[1] = g_pinned.begin()->second;
+}
 API void t_refuse_pins(int on) { g_refuse_pins = on; }
 }

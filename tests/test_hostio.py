@@ -215,3 +215,22 @@ def test_a_pool_that_gets_no_slots_leaves_the_plain_copy(host):
     host.lib.t_refuse_pins(0)
     assert host.down(h, 8 * MB)["pinned_copies"] == 0
     host.lib.t_close(h)
+
+
+def test_pinned_memory_is_not_inherited_by_child_processes(host):
+    """A fork must not turn the pages that the device knows into copies: the
+    mapping carries the kernel's do-not-copy flag."""
+    h = host.open(8 * 1000)
+    out = (C.c_size_t * 2)()
+    host.lib.t_some_pinned(out)
+    start, size = out
+    flags = None
+    for line in Path("/proc/self/smaps").read_text().splitlines():
+        head = line.split()[0]
+        if "-" in head and not head.endswith(":"):
+            lo, hi = (int(x, 16) for x in head.split("-"))
+            inside = lo <= start and start + size <= hi
+        elif head == "VmFlags:" and inside:
+            flags = line.split()[1:]
+    assert flags is not None and "dc" in flags
+    host.lib.t_close(h)
