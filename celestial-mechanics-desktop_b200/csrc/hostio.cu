@@ -53,12 +53,14 @@ constexpr size_t kRowAlign = 256;
 // 5.7 / 2.2).
 constexpr size_t kPoolUp = 28 << 20, kPoolDown = 2 << 20;
 // The slots come once a program has moved this much by plain copies: one that
-// moves less never pays for them.  They come a few at a time, so that no call is
-// held up by more than 2 to 3 ms, and the six after it by 1.3 (all 16 MB at once
-// took 7 to 10, and up to 20 on another host).
+// moves less never pays for them.  They come a few at a time, so that the call
+// that gets the first (and the threads) is held up by some 2 ms and the six after
+// it by 0.6 (all 16 MB at once by cudaHostAlloc took 7 to 20).
 constexpr size_t kPoolAfter = 32 << 20;
-constexpr int kFirstSlots = 4, kMoreSlots = 2;
-constexpr size_t kPage = 4096;
+constexpr int kBlockSlots = 2;  // pinned together: one huge page
+constexpr int kFirstSlots = 2 * kBlockSlots, kMoreSlots = kBlockSlots;
+static_assert(kSlots % kBlockSlots == 0, "whole blocks");
+constexpr size_t kPage = 4096, kHugePage = 2 << 20, kHugeFrom = 512 << 10;
 constexpr size_t kMaxSpare = 8;
 
 // A handle's pinned memory: two halves and kHostExtra bytes.
@@ -73,29 +75,44 @@ struct Chunk {
     size_t bytes;
 };
 
-// Pinned memory as ordinary pages that are registered: 0.4 ms for the 230 KB
-// of a 1,000-body handle, 1 ms for 1 MB, where cudaHostAlloc takes 1.3 to 3 ms
-// for either unless other pinned memory is about (ms to create a handle for
+// Pinned memory as ordinary pages that are registered, huge ones from kHugeFrom
+// bytes on: 0.4 to 0.7 ms for the 230 KB of a 1,000-body handle, 0.45 ms for 1 or
+// 2 MB (1.3 and 2 without huge pages), where cudaHostAlloc takes 1.3 to 3 ms for
+// any of them unless other pinned memory is about (ms to create a handle for
 // 1,000 bodies: 4.2 without pinned memory, 4.9 so, 6.5 that way).  A child process
 // does not inherit them: a fork would otherwise have the parent write to copies
 // of the pages while the device keeps to the old ones, where the kernel does
 // not look after registered pages itself.
+size_t mapped(size_t bytes) {
+    return bytes < kHugeFrom ? bytes : (bytes + kHugePage - 1) / kHugePage * kHugePage;
+}
+
 char* pin(size_t bytes) {
-    void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    const size_t size = mapped(bytes);
+    const size_t slack = bytes < kHugeFrom ? 0 : kHugePage;  // to start at a huge page
+    char* p = (char*)mmap(nullptr, size + slack, PROT_READ | PROT_WRITE,
+                          MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
     if (p == MAP_FAILED) return nullptr;
-    if (madvise(p, bytes, MADV_DONTFORK) != 0 ||
+    if (slack) {
+        const size_t head = (kHugePage - (size_t)p % kHugePage) % kHugePage;
+        if (head) munmap(p, head);
+        if (slack > head) munmap(p + head + size, slack - head);
+        p += head;
+        madvise(p, size, MADV_HUGEPAGE);  // where the kernel has none: small pages
+    }
+    if (madvise(p, size, MADV_DONTFORK) != 0 ||
         cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) {
         cudaGetLastError();
-        munmap(p, bytes);
+        munmap(p, size);
         return nullptr;
     }
-    return (char*)p;
+    return p;
 }
 
 void unpin(char* p, size_t bytes) {
     if (!p) return;
     cudaHostUnregister(p);
-    munmap(p, bytes);
+    munmap(p, mapped(bytes));
 }
 
 size_t pin_bytes(size_t half) { return 2 * half + kHostExtra; }
@@ -187,20 +204,21 @@ struct CopyPool {
         }
     }
 
-    // `count` more slots (busy held).
+    // `count` more slots, in blocks (busy held).
     void grow(int count) {
         // another thread of the program may be capturing a graph
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
-        for (; count > 0 && slots < kSlots && !full; count--) {
-            buf[slots] = pin(kSlotBytes);
-            if (buf[slots] &&
-                cudaEventCreateWithFlags(&ev[slots], cudaEventDisableTiming) == cudaSuccess) {
-                slots++;
+        for (; count > 0 && slots < kSlots && !full; count -= kBlockSlots) {
+            char* block = pin(kBlockSlots * kSlotBytes);
+            bool ok = block != nullptr;
+            for (int k = slots; ok && k < slots + kBlockSlots; k++)
+                ok = ev[k] || cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming) == cudaSuccess;
+            if (ok) {
+                for (int k = 0; k < kBlockSlots; k++) buf[slots++] = block + k * kSlotBytes;
             } else {
                 cudaGetLastError();
-                unpin(buf[slots], kSlotBytes);
-                buf[slots] = nullptr;
+                unpin(block, kBlockSlots * kSlotBytes);
                 full = true;
             }
         }
@@ -277,7 +295,7 @@ void pool_destroy(CopyPool* p) {
             cudaEventDestroy(p->ev[k]);
         }
     for (const PinBuf& b : p->spare) unpin(b.p, pin_bytes(b.half));
-    for (char* b : p->buf) unpin(b, kSlotBytes);
+    for (int k = 0; k < p->slots; k += kBlockSlots) unpin(p->buf[k], kBlockSlots * kSlotBytes);
     delete p;
 }
 
