@@ -408,7 +408,8 @@ NB_API int32_t nb_ens_info(const nb_ensemble* h, int64_t* out, int32_t n);
 NB_API int32_t nb_ens_set_param_f64(nb_ensemble* h, int32_t param, double value);
 NB_API int32_t nb_ens_set_param_i32(nb_ensemble* h, int32_t param, int32_t value);
 /* Positions, velocities, masses; accelerations are unknown until the first
- * force evaluation (nb_ens_step does one first when needed). */
+ * force evaluation (nb_ens_step does one first when needed).  A call refused
+ * with NB_ERR_NONFINITE leaves the state as it was. */
 NB_API int32_t nb_ens_set_state(nb_ensemble* h, const double* px, const double* py,
                                 const double* pz, const double* vx, const double* vy,
                                 const double* vz, const double* mass);
