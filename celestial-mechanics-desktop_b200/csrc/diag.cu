@@ -86,7 +86,7 @@ k_diag_final(int nblocks, const double* __restrict__ part, int n_items,
 // correctly rounded square root and division per pair, left the first rows'
 // blocks running alone.  A whole diagnostics call, before -> now: 2,000
 // bodies 444 -> 54 us, 65,537 bodies 13.39 -> 2.00 ms, 131,072 bodies 29.3 ->
-// 7.9 ms (1, 3 and 4 rows per thread were within 5 %).
+// 7.9 ms (the FP64 pipe is 74 % busy; 1, 3 and 4 rows per thread were within 5 %).
 constexpr int kPeThreads = 256;
 constexpr int kPeRows = 2;                        // rows per thread
 constexpr int kPeTile = kPeThreads * kPeRows;     // rows per item
